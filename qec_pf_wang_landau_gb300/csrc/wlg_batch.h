@@ -20,7 +20,7 @@ namespace wlg {
 // ---- kernels (wlg_engine.cu)
 wlg_status launch_pre_batch(const PreDesc* d_descs, int n, int threads, int smem, int8_t* Jpool, uint8_t* seen_pool,
                             int8_t* found_pool, int* fflag_pool, cudaStream_t s);
-// variant: kernel_variant (form | kKernelRows)
+// variant: kernel_variant
 int main_batch_capacity(int variant, int cta_threads, int smem);
 wlg_status launch_main_batch(int variant, const MainDesc* d_descs, const int* d_order, int n, int team_size,
                              int team_bytes, int teams_per_cta, int grid, int* d_next, double* gpool,
@@ -90,6 +90,12 @@ struct Exec {
   virtual ~Exec() = default;
   // device buffer for `slot` of at least `bytes` bytes
   virtual wlg_status buffer(Slot slot, size_t bytes, void** out) = 0;
+  // bytes that buffer(slot) could be given now, when that is limited
+  virtual size_t available(Slot slot)
+  {
+    (void)slot;
+    return ~size_t{0} >> 1;
+  }
 };
 
 inline wlg_status fail(Exec& ex, wlg_status st, const std::string& msg)
@@ -166,35 +172,63 @@ wlg_status handoff(Exec& ex, const wlg_problem* probs, int n, wlg_result* result
 wlg_status prepare_batch(Exec& ex, const wlg_problem* probs, int n, wlg_result* results, Prepared& prep, Handoff& ho,
                          const int8_t* couplings = nullptr, const unsigned char* given = nullptr);
 
-// Main-run forms by lattice storage: 0 spins in shared memory, 1 spins in a
-// register, 2 register spins + neighbour table (X, Y >= 3), 3 as 0 with
-// FP64 log g in global memory (teams whose state exceeds shared memory).
-// (Spins of 65-256-site lattices in 2-4 register words with a neighbour
-// table were built and measured: 3-7 % slower than form 0, whose loads are
-// broadcasts or conflict-free columns.)
+// A main-run kernel: how it keeps the lattice (Store), plus where FP64 log g
+// and the histogram live and whether the team does without guard bins and ring.
+constexpr int kVariantGlobal = 8;  // log g and histogram in global memory
+constexpr int kVariantTight = 16;  // see team_layout; always with kVariantGlobal
 constexpr int kSmemBytes = 227 * 1024;
 
-inline int main_form(const MainDesc& d) { return d.N > 64 ? 0 : (d.X >= 3 && d.Y >= 3 ? 2 : 1); }
+inline int variant_store(int variant) { return variant & 7; }
 
-// Shared-memory bytes of a team running d in form `form`.
-inline int team_bytes(const MainDesc& d, int form, int team)
+// The form wlg.h reports: 0 lattice and log g in shared memory, 1 lattice in a
+// register, 2 the register with a neighbour table, 3 log g in global memory.
+inline int variant_form(int variant)
 {
-  const bool reg = form == 1 || form == 2;
-  return align16(team_layout(team, d.L, d.nwL, d.nwM, d.I, reg ? 2 : d.nwL, form == 2 ? d.N : 0, form != 3).bytes +
-                 16);
+  if ((variant & kVariantGlobal) != 0) return 3;
+  const int s = variant_store(variant);
+  return s == kStoreReg || s == kStoreTable ? s : 0;
 }
 
-// The form d runs in: main_form, or FP64 log g in global memory when the
-// shared-memory lattice form's state does not fit.
-inline int fit_form(const MainDesc& d, int team)
+// Shared-memory bytes of a team running d in `variant`.
+inline int team_bytes(const MainDesc& d, int variant, int team)
 {
-  const int form = main_form(d);
-  return form == 0 && team_bytes(d, 0, team) > kSmemBytes ? 3 : form;
+  return align16(
+    team_layout(d, team, variant_store(variant), (variant & kVariantGlobal) != 0, (variant & kVariantTight) != 0).bytes +
+    16);
 }
 
-// The kernel of a main-run launch: its form (fit_form, 0-3) plus
-// kKernelRows when its problems keep lattices one row per word
-// (lattice_rows; forms 0 and 3 only).  Problems of one launch share both.
-inline int kernel_variant(const MainDesc& d, int team) { return fit_form(d, team) | (d.rows != 0 ? kKernelRows : 0); }
+// The lattice storage of d: registers up to 64 sites, else bonds where a row's
+// right and down bonds fit one word (Y <= 16: two words read per proposal
+// instead of three rows and three couplings), else rows, else linear words.
+// Tight states keep rows, whose tables take no room.
+inline int lattice_store(const MainDesc& d, bool tight)
+{
+  if (d.N <= 64) return d.X >= 3 && d.Y >= 3 ? kStoreTable : kStoreReg;
+  if (d.rows == 0) return kStoreLinear;
+  return d.Y <= 16 && !tight ? kStoreBonds : kStoreRows;
+}
+
+inline int tight_variant(const MainDesc& d) { return lattice_store(d, true) | kVariantGlobal | kVariantTight; }
+
+// Bytes that decide whether a problem is taken at all: 8 per bin and walker
+// (16 for lattices in registers) plus the lattice must fit one SM.
+inline int admission_bytes(const MainDesc& d, int team)
+{
+  const int store = lattice_store(d, true);
+  const bool reg = store == kStoreReg || store == kStoreTable;
+  return team_bytes(d, tight_variant(d), team) +
+         (reg ? 8 * d.L * team - (store == kStoreTable ? align16(4 * d.N) : 0) : 0);
+}
+
+// The kernel of d: everything in shared memory where it fits, else log g and
+// the histogram in global memory (read and written once per sweep), else the
+// tight layout.  Problems of one launch share it.
+inline int kernel_variant(const MainDesc& d, int team)
+{
+  const int store = lattice_store(d, false);
+  if (team_bytes(d, store, team) <= kSmemBytes) return store;
+  if (team_bytes(d, store | kVariantGlobal, team) <= kSmemBytes) return store | kVariantGlobal;
+  return tight_variant(d);
+}
 
 }  // namespace wlg

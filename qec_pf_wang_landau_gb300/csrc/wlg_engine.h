@@ -46,8 +46,6 @@ struct PreDesc {
 // -1 coupling; right bonds (site, site + 1 in the row) and down bonds (site,
 // site + Y) are packed the same way as the sites that own them.
 WLG_HD inline bool lattice_rows(int X, int Y) { return X * Y > 64 && Y >= 2 && Y <= 32; }
-// bit of a main-run kernel variant (kernel_variant) for the row layout
-constexpr int kKernelRows = 4;
 WLG_HD inline int lattice_words(int X, int Y) { return lattice_rows(X, Y) ? X : (X * Y + 31) / 32; }
 // word and bit of site q (q = i*Y + j)
 WLG_HD inline void lattice_bit(int X, int Y, int q, int& word, int& bit)
@@ -137,44 +135,70 @@ WLG_HD inline StateLayout state_layout(int P, int I, int nwL, int L)
   return s;
 }
 
+// How a main-run kernel keeps the lattice.  Spins: linear shared words, one u64
+// register (N <= 64), the register with a neighbour table (X, Y >= 3), or one
+// row per shared word (lattice_rows).  Bonds: for rows of up to 16 sites, the
+// unsatisfied right bonds (low half) and down bonds (high half) of a row in one
+// word instead of its spins.
+enum Store { kStoreLinear = 0, kStoreReg = 1, kStoreTable = 2, kStoreRows = 3, kStoreBonds = 4 };
+
+// Draws a walker keeps ahead (a power of two), and the bytes of a warp's ring
+// of them: slot after slot of 32 lanes, the first slot repeated at the end.
+constexpr int kRingSlots = 16;
+constexpr int kRingWarpBytes = (kRingSlots + 1) * 32 * 4;
+
+// Energies a proposal can lie beyond its window: one flip changes the energy
+// by at most 8.
+WLG_HD inline int guard_bins(int lg) { return 8 >> lg; }
+
 // Team shared-memory layout of a problem (bytes, 16-byte aligned pieces).
 struct TeamLayout {
-  int off_G, off_Gf, off_H, off_lat, off_E, off_perm, off_mask, off_J, off_nbt, off_f, off_cond, off_flat, off_stab,
-    off_win, off_misc;
+  int off_G, off_H, off_pair, off_ring, off_lat, off_E, off_perm, off_mask, off_J, off_tab, off_f, off_cond, off_flat,
+    off_stab, off_win, off_misc;
   int bytes;
 };
 
 WLG_HD inline int align16(int x) { return (x + 15) & ~15; }
 
-// reg_lattice: spins in a register (N <= 64); nbt_sites: sites of the
-// neighbour table (0 when the table is not used); g_in_smem: FP64 log g in
-// shared memory (else in a global pool).
-// lat_words: 32-bit words per walker of the lattice area (the lattice
-// itself, or the exchange staging of a register lattice); nbt_entries:
-// 16-byte neighbour-table entries.
-WLG_HD inline TeamLayout team_layout(int team, int L, int nwL, int nwM, int I, int lat_words, int nbt_entries,
-                                     bool g_in_smem = true)
+// What a team keeps at the start of its shared memory: the problem, and where
+// its pieces lie (values used between sweeps would otherwise hold registers
+// through them).
+struct TeamHead {
+  MainDesc d;
+  TeamLayout lay;
+  StateLayout state;
+};
+constexpr int kTeamHeadBytes = static_cast<int>((sizeof(TeamHead) + 15) & ~size_t{15});
+
+// global_g: FP64 log g and the histogram live in global memory.  tight: no
+// guard bins and no draw ring, for states that would not fit otherwise.
+WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, bool global_g, bool tight)
 {
+  const bool reg = store == kStoreReg || store == kStoreTable;
+  const int L = d.L, I = d.I;
+  const int rows = tight ? L : L + 2 * guard_bins(d.lg);
   TeamLayout t{};
-  int o = 0;
+  int o = tight ? 0 : kTeamHeadBytes;
   t.off_G = o;
-  o = align16(o + (g_in_smem ? 8 * L * team : 0));
-  t.off_Gf = o;
-  o = align16(o + 4 * L * team);
+  o = align16(o + (global_g ? 0 : 8 * L * team));
   t.off_H = o;
-  o = align16(o + 4 * L * team);
-  t.off_lat = o;
-  o = align16(o + 4 * lat_words * team);
+  o = align16(o + (global_g ? 0 : 4 * L * team));
+  t.off_pair = o;  // {float shadow of log g, visits} per bin, guard bins included
+  o = align16(o + 8 * rows * team);
+  t.off_ring = o;
+  o = align16(o + (tight ? 0 : team / 32 * kRingWarpBytes));
+  t.off_lat = o;  // the lattice, or the exchange staging of a register lattice
+  o = align16(o + 4 * (reg ? 2 : d.nwL) * team);
   t.off_E = o;
   o = align16(o + 4 * team);
   t.off_perm = o;
   o = align16(o + 4 * team);
   t.off_mask = o;
-  o = align16(o + 4 * nwM);
+  o = align16(o + 4 * d.nwM);
   t.off_J = o;
-  o = align16(o + 4 * 2 * nwL);
-  t.off_nbt = o;
-  o = align16(o + 16 * nbt_entries);
+  o = align16(o + 4 * 2 * d.nwL);
+  t.off_tab = o;  // neighbour table and degrees per site, or bond masks per column and per row
+  o = align16(o + (store == kStoreTable ? 20 * d.N : (store == kStoreBonds ? align16(8 * d.Y) + 16 * d.X : 0)));
   t.off_f = o;  // f [I], then ln f [I]
   o = align16(o + 16 * I);
   t.off_cond = o;

@@ -331,6 +331,12 @@ struct ContextExec final : Exec {
     *out = ctx->buf[slot].p;
     return st;
   }
+  size_t available(Slot slot) override
+  {
+    if (ctx->budget == 0) return Exec::available(slot);
+    const size_t others = ctx->used - ctx->buf[slot].cap;
+    return ctx->budget > others ? ctx->budget - others : 0;
+  }
 };
 
 }  // namespace
@@ -703,6 +709,10 @@ wlg_status prepare_batch(Exec& ex, const wlg_problem* probs, int n, wlg_result* 
 
 namespace {
 
+// Doubles of a resident team's slice of the global pool: FP64 log g [L][team],
+// then the histogram (32 bits) [L][team].
+long long pool_slice(int L, int team) { return (3LL * L * team + 1) / 2; }
+
 constexpr int kTimedEpoch = 4;  // outer iterations per launch under a time limit
 
 // The main run of a prepared batch: one persistent launch per (form, team
@@ -757,10 +767,12 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     int bytes = 0;
     int Lmax = 1;
     for (int i : idx) {
-      bytes = std::max(bytes, wlg::team_bytes(prep.main[i], variant & 3, team));
+      bytes = std::max(bytes, wlg::team_bytes(prep.main[i], variant, team));
       Lmax = std::max(Lmax, prep.main[i].L);
     }
-    if (bytes > wlg::kSmemBytes) return fail(ex, WLG_ERR_INVALID, "problem state exceeds shared memory");
+    for (int i : idx)
+      if (wlg::admission_bytes(prep.main[i], team) > wlg::kSmemBytes)
+        return fail(ex, WLG_ERR_INVALID, "problem state exceeds shared memory");
     int per_cta = team <= 256 ? 256 / team : 1;
     per_cta = std::min(per_cta, (227 * 1024) / bytes);
     if (team > 32) per_cta = std::min(per_cta, 15);
@@ -803,9 +815,16 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   if ((st = ex.buffer(kRes, static_cast<size_t>(m) * sizeof(MainResult), &d_res)) != WLG_OK) return st;
   if ((st = ex.buffer(kNext, launches.size() * sizeof(int), &d_next)) != WLG_OK) return st;
   if (timed) cudaMemsetAsync(d_res, 0, static_cast<size_t>(m) * sizeof(MainResult), ex.stream);
-  // grids, and the global log g pool of the variant-3 launches (one slice per
-  // resident team, launches side by side)
+  // grids, and the pool of the launches that keep log g and the histogram in
+  // global memory (one slice per resident team, launches side by side; the
+  // saved state holds them in resumable runs)
   std::vector<int> grids(launches.size());
+  std::vector<long long> pool_later(launches.size() + 1, 0);  // one CTA's slices of each later launch
+  for (size_t g = launches.size(); g-- > 1;) {
+    const bool global = (std::get<0>(launches[g]) & wlg::kVariantGlobal) != 0;
+    const long long cta = std::get<3>(launches[g]) * pool_slice(std::get<6>(launches[g]), std::get<1>(launches[g]));
+    pool_later[g - 1] = pool_later[g] + (global ? cta : 0);
+  }
   std::vector<long long> gpool_off(launches.size(), 0);
   long long gpool_doubles = 0;
   for (size_t g = 0; g < launches.size(); ++g) {
@@ -813,9 +832,15 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     const int cap = wlg::main_batch_capacity(variant, team * per_cta, bytes * per_cta);
     if (cap <= 0) return fail(ex, WLG_ERR_CUDA, "main-run configuration does not fit an SM");
     grids[g] = std::min(cap, (count + per_cta - 1) / per_cta);
-    if ((variant & 3) == 3) {
+    if ((variant & wlg::kVariantGlobal) != 0 && !timed) {
+      // a fixed arena or a budget may not hold a slice for every team that
+      // the GPU could hold: fewer resident teams then take the problems in turn
+      const long long slice = pool_slice(Lmax, team);
+      const long long room = static_cast<long long>(ex.available(kGpool) / sizeof(double)) - gpool_doubles;
+      const long long later = pool_later[g];
+      grids[g] = static_cast<int>(std::max(1LL, std::min<long long>(grids[g], (room - later) / (slice * per_cta))));
       gpool_off[g] = gpool_doubles;
-      gpool_doubles += static_cast<long long>(grids[g]) * per_cta * Lmax * team;
+      gpool_doubles += grids[g] * per_cta * slice;
     }
   }
   void* d_gpool = nullptr;
@@ -835,16 +860,16 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     for (size_t g = 0; g < launches.size() && s2 == WLG_OK; ++g) {
       const auto [variant, team, bytes, per_cta, first, count, Lmax] = launches[g];
       const int grid = grids[g];
-      double* gp = (variant & 3) == 3 ? static_cast<double*>(d_gpool) + gpool_off[g] : nullptr;
+      double* gp = (variant & wlg::kVariantGlobal) != 0 && !timed ? static_cast<double*>(d_gpool) + gpool_off[g] : nullptr;
       s2 = wlg::launch_main_batch(
         variant, static_cast<const MainDesc*>(d_md), static_cast<const int*>(d_order) + first, count, team, bytes,
-        per_cta, grid, static_cast<int*>(d_next) + g, gp, static_cast<long long>(Lmax) * team,
+        per_cta, grid, static_cast<int*>(d_next) + g, gp, pool_slice(Lmax, team),
         static_cast<const uint32_t*>(d_Jw), static_cast<const uint32_t*>(d_latw), static_cast<const int*>(d_win),
         static_cast<const uint32_t*>(d_mask), static_cast<double*>(d_out), static_cast<MainResult*>(d_res),
         static_cast<unsigned char*>(d_state), n_fork > 0 ? ex.aux[g % n_fork] : ex.stream);
       if (s2 == WLG_OK) {
         ++ex.launches;
-        ex.main_forms |= 1 << (variant & 3);
+        ex.main_forms |= 1 << wlg::variant_form(variant);
       }
     }
     for (int a = 0; a < n_fork; ++a) {  // join (also after a failed launch)
@@ -1323,7 +1348,7 @@ wlg_status wlg_context_autotune(wlg_context* ctx, const wlg_problem* problems, i
         sub.main_problem.push_back(prep.main_problem[i]);
       }
       const int limit = key.second <= 256 ? 256 / key.second : 1;
-      wlg_tuning t{key.first & 3, key.second, 1, 0.0f, 0};
+      wlg_tuning t{variant_form(key.first), key.second, 1, 0.0f, 0};
       float best_ms = 0.0f;
       for (int c = 1; c <= limit; c *= 2) {
         const std::map<std::pair<int, int>, int> force{{key, c}};
@@ -1421,6 +1446,7 @@ wlg_status wlg_class_log_probs(const int* energies, const double* log_g, const l
 
 namespace wlg {
 wlg_status noalloc_arena(void** out, size_t* bytes);
+size_t noalloc_admitted();
 }
 
 namespace {
@@ -1439,7 +1465,7 @@ struct ArenaExec final : Exec {
     }
     const size_t off = (used + 255) & ~size_t{255};
     if (off + bytes > cap) {
-      err = "batch does not fit the " + std::to_string(cap >> 20) + " MiB no-allocation arena";
+      err = "batch does not fit the no-allocation arena";
       return WLG_ERR_CAPACITY;
     }
     slot_ptr[slot] = base + off;
@@ -1448,16 +1474,21 @@ struct ArenaExec final : Exec {
     *out = slot_ptr[slot];
     return WLG_OK;
   }
+  size_t available(Slot slot) override
+  {
+    const size_t off = (used + 255) & ~size_t{255};
+    return std::max(slot_cap[slot], cap > off ? cap - off : 0);
+  }
 };
 
 // Upper bound of the arena bytes a batch needs, from the problem parameters
 // alone (windows of the full range [-2N, 2N], energy step 2), so oversized
-// batches are rejected before anything runs.  This includes the global log g
-// pool of the form-3 launches (run_main): one slice of L x team doubles per
-// resident team, at most (problems + teams per CTA - 1) slices per launch (one
-// launch per team size and lattice layout), counted for every problem whose
-// full-range state would not fit shared memory (its real windows are never
-// wider, so no form-3 problem is missed).
+// batches are rejected before anything runs.  This includes L x team doubles of
+// global log g, at most (problems + teams per CTA - 1) times per launch (one
+// launch per team size and lattice layout), for every problem whose full-range
+// state of 16 bytes per bin and walker would not fit shared memory.  The pool
+// that run_main then takes follows the room left (Exec::available); one CTA's
+// slices fit in the part of the arena beyond the admitted bytes.
 size_t noalloc_bound(const wlg_problem* probs, int n)
 {
   auto pad = [](size_t x) { return (x + 255) & ~size_t{255}; };
@@ -1477,8 +1508,11 @@ size_t noalloc_bound(const wlg_problem* probs, int n)
     d.L = static_cast<int>(nbins);
     d.nwL = static_cast<int>(nwL);
     d.nwM = static_cast<int>((nbins + 31) / 32);
+    d.rows = wlg::lattice_rows(q.X, q.Y) ? 1 : 0;
+    d.lg = 1;
     const int team = wlg::round32(q.intervals * q.walkers_per_interval);
-    if (wlg::fit_form(d, team) == 3) {
+    const size_t state = static_cast<size_t>(wlg::admission_bytes(d, team)) + 8 * nbins * static_cast<size_t>(team);
+    if (N > 64 && state > static_cast<size_t>(wlg::kSmemBytes)) {
       auto& e = pool[{team, wlg::lattice_rows(q.X, q.Y)}];
       e.first += 1;
       e.second = std::max(e.second, nbins);
@@ -1522,7 +1556,7 @@ wlg_status wlg_solve_raw_noalloc(const wlg_problem* problems, int n, wlg_result*
     wlg_status st = wlg::noalloc_arena(&base, &ex.cap);
     if (st != WLG_OK) return st;
     ex.base = static_cast<unsigned char*>(base);
-    if (noalloc_bound(problems, n) > ex.cap) return WLG_ERR_CAPACITY;
+    if (noalloc_bound(problems, n) > wlg::noalloc_admitted()) return WLG_ERR_CAPACITY;
     cudaGetDevice(&ex.device);
     ex.stream = wlg::as_stream(stream);
     std::vector<MainResult> mres;
