@@ -18,6 +18,7 @@
 #include "wlg_internal.h"
 #include "wlg_lattice.cuh"
 #include "wlg_main_fn.h"
+#include "wlg_pre.cuh"
 #include "wlg_rng.cuh"
 
 namespace wlg {
@@ -25,30 +26,115 @@ namespace {
 
 // ------------------------------------------------------------ pre-run -----
 
-// Site of a draw: trunc(double(u) * ((N-1) + 0.999999)) (wl.cu:63-65).  With
-// f = x / 2^32 the reference's product lies within N*2^-23 + 1e-6 of f*N, so
-// floor(f*N) = umulhi(x, N) is exact unless the fraction x*N mod 2^32 lies
-// within site_thr (= 2^32 (N 2^-21 + 2^-18), >= 4x that bound) of an
-// integer; there the reference's own float/double expression below decides.
-// No int<->float conversion on the common path (they share GB300's slow
-// FP64 pipe).  Out of line: inlined, its FP64 multiply and conversions would
-// be scheduled into every step.
-__device__ __noinline__ int site_exact(uint32_t x, double scale)
+// Draws, in {-1, 1}: the couplings of a sample with its error chain
+// (wl.cu:364-428, prerun.cu:56-75) and the lattice every walker starts from
+// (wl.cu:430-457, CAS winner fixed to site 0).
+__device__ __forceinline__ int8_t draw_coupling(const PreDesc& d, const int8_t* __restrict__ Jpool, int q)
 {
-  return static_cast<int>(trunc(static_cast<double>(unit_float(x)) * scale));
+  int8_t v;
+  if (d.given_J) {
+    v = Jpool[d.off_J + q];
+  } else {
+    Stream st;
+    st.init(key_size(d.seed, static_cast<uint64_t>(d.sample)), 0, static_cast<uint64_t>(q));
+    const double u = st.uniform();
+    v = (u < d.prob) ? -1 : 1;
+  }
+  const bool h = d.error_class == 'h' || d.error_class == 'c', vert = d.error_class == 'v' || d.error_class == 'c';
+  if (h && q >= d.N && q < d.N + d.Y) v = static_cast<int8_t>(-v);
+  if (vert && q < d.N && q % d.Y == 0) v = static_cast<int8_t>(-v);
+  return v;
 }
 
-__global__ void __launch_bounds__(1024) k_pre_batch(const PreDesc* __restrict__ descs, int n,
-                                                    int8_t* __restrict__ Jpool, uint8_t* __restrict__ seen_pool,
-                                                    int8_t* __restrict__ found_pool, int* __restrict__ fflag_pool)
+__device__ __forceinline__ int8_t draw_spin(const PreDesc& d, int q)
 {
-  const int p = blockIdx.x;
-  if (p >= n) return;
-  const PreDesc d = descs[p];
+  const uint64_t key = key_u32(d.seed, static_cast<uint64_t>(d.sample));
+  Stream st;
+  st.init(key, 1, 0);
+  const float p0 = st.uniform();
+  st.init(key, 1, static_cast<uint64_t>(q) + 1);
+  const double u = st.uniform();
+  return (u < p0) ? -1 : 1;
+}
+
+// The whole pre-run of one problem on bond words.
+template <bool kTwo>
+__device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* smem, int8_t* __restrict__ Jpool,
+                                            uint8_t* __restrict__ seen_pool, int8_t* __restrict__ found_pool,
+                                            int* __restrict__ fflag_pool)
+{
+  constexpr int kW = kTwo ? 2 : 1;
+  const int N = d.N, X = d.X, Y = d.Y, L = 4 * N + 1, tid = threadIdx.x;
+  const int threads = (d.walkers + 31) / 32 * 32, Lh = pre_hist_words(L);
+  if (tid >= threads) return;  // warps beyond this problem's walkers
+  const PreLayout l = pre_layout(X, Y, L, d.n_int, threads);
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + l.off_hist);
+  uint32_t* thr = reinterpret_cast<uint32_t*>(smem + l.off_thr);
+  uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
+  uint32_t* base = reinterpret_cast<uint32_t*>(smem + l.off_base);
+  uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
+  uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
+  PreWalk p{X, Y, d.boundary, -2 * N, 2 * N, d.n_int, d.len_int, d.n_iter, threads, hist,
+            reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr,
+            col, row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words), found_pool + d.off_found};
+  const PreSync sync{threads};
+  for (int q = tid; q < 2 * Lh; q += threads) hist[q] = 0;
+  for (int q = tid; q < d.n_int; q += threads) {
+    p.claim[q] = kPreEmpty;
+    p.found_E[q] = 0;
+  }
+  for (int q = tid; q < X; q += threads) Jr[q] = Jr[X + q] = base[q] = 0;
+  fill_accept(thr, tid);
+  fill_bonds<kTwo>(col, row, X, Y, d.boundary, tid, threads);
+  sync();
+  for (int q = tid; q < 2 * N; q += threads) {
+    const int8_t v = draw_coupling(d, Jpool, q);
+    const int s = q < N ? q : q - N, i = s / Y;
+    if (v < 0) atomicOr(&Jr[(q < N ? 0 : X) + i], 1u << (s - i * Y));
+    Jpool[d.off_J + q] = v;
+  }
+  for (int q = tid; q < N; q += threads) {
+    const int i = q / Y;
+    if (draw_spin(d, q) < 0) atomicOr(&base[i], 1u << (q - i * Y));
+  }
+  sync();
+  const int w = tid;
+  uint32_t unsat = 0;
+  for (int i = 0; i < X; ++i) {
+    uint32_t h, v = 0;
+    bond_words<kTwo>(base[i], base[i + 1 < X ? i + 1 : 0], Jr[i], Jr[X + i], Y, d.boundary != 0, i + 1 == X, h, v);
+    p.words[i * kW * threads + w] = h;
+    unsat += __popc(h);
+    if constexpr (kTwo) {
+      p.words[(i * kW + 1) * threads + w] = v;
+      unsat += __popc(v);
+    }
+  }
+  // wl.cu:261-340: minus the sum over bonds of s s J
+  const int bonds = d.boundary == 0 ? 2 * N : 2 * N - X - Y;
+  int E = 2 * static_cast<int>(unsat) - bonds;
+  uint32_t s0 = base[0] & 1u;
+  uint64_t pos = 0;
+  pre_walk<kTwo, false>(p, sync, w, w < d.walkers, key_u32(d.seed, static_cast<uint64_t>(d.sample)),
+                        2 + static_cast<uint64_t>(w), pos, E, s0);
+  for (int q = tid; q < L; q += threads) seen_pool[d.off_seen + q] = hist[q] != 0 ? 1 : 0;
+  for (int q = tid; q < d.n_int; q += threads) {
+    const bool found = p.claim[q] != kPreEmpty;
+    fflag_pool[d.off_fflag + q] = found ? 1 : 0;
+    fflag_pool[d.off_fflag + d.n_int + q] = found ? p.found_E[q] : 0;
+  }
+}
+
+// The whole pre-run on int8 lattices, 64-bit counts and two barriers a round:
+// rows of more than 32 sites, 2^31 visits and more, and bond words too large
+// for shared memory.
+__device__ __forceinline__ void pre_problem_i8(const PreDesc& d, unsigned char* smem, int8_t* __restrict__ Jpool,
+                                               uint8_t* __restrict__ seen_pool, int8_t* __restrict__ found_pool,
+                                               int* __restrict__ fflag_pool)
+{
   const int N = d.N, X = d.X, Y = d.Y;
   const int L = 4 * N + 1;
   const int e_min = -2 * N;
-  extern __shared__ __align__(16) unsigned char smem[];
   unsigned long long* hist = reinterpret_cast<unsigned long long*>(smem);
   int* claim = reinterpret_cast<int*>(hist + L);
   int* found = claim + d.n_int;
@@ -57,40 +143,19 @@ __global__ void __launch_bounds__(1024) k_pre_batch(const PreDesc* __restrict__ 
   int8_t* lat = J + 2 * N;  // [walkers][N]
 
   const int tid = threadIdx.x;
-  // disorder (wl.cu:364-386), or the caller's pattern, and the error chain
-  // (wl.cu:388-428, prerun.cu:56-75)
   for (int q = tid; q < 2 * N; q += blockDim.x) {
-    if (d.given_J) {
-      J[q] = Jpool[d.off_J + q];
-      continue;
-    }
-    Stream st;
-    st.init(key_size(d.seed, static_cast<uint64_t>(d.sample)), 0, static_cast<uint64_t>(q));
-    const double u = st.uniform();
-    J[q] = (u < d.prob) ? -1 : 1;
+    J[q] = draw_coupling(d, Jpool, q);
+    Jpool[d.off_J + q] = J[q];
   }
   for (int q = tid; q < L; q += blockDim.x) hist[q] = 0;
   for (int q = tid; q < d.n_int; q += blockDim.x) {
     claim[q] = INT_MAX;
     found[q] = 0;
   }
+  for (int q = tid; q < N; q += blockDim.x) lat[q] = draw_spin(d, q);
+  __shared__ uint32_t acc_thr[kAcceptEntries];
+  fill_accept(acc_thr, tid);
   __syncthreads();
-  if (d.error_class == 'h' || d.error_class == 'c')
-    for (int q = tid; q < Y; q += blockDim.x) J[N + q] = static_cast<int8_t>(-J[N + q]);
-  if (d.error_class == 'v' || d.error_class == 'c')
-    for (int q = tid; q < X; q += blockDim.x) J[q * Y] = static_cast<int8_t>(-J[q * Y]);
-  // lattice (wl.cu:430-457, CAS winner fixed to site 0)
-  const uint64_t key_l = key_u32(d.seed, static_cast<uint64_t>(d.sample));
-  for (int q = tid; q < N; q += blockDim.x) {
-    Stream st;
-    st.init(key_l, 1, 0);
-    const float p0 = st.uniform();
-    st.init(key_l, 1, static_cast<uint64_t>(q) + 1);
-    const double u = st.uniform();
-    lat[q] = (u < p0) ? -1 : 1;
-  }
-  __syncthreads();
-  for (int q = tid; q < 2 * N; q += blockDim.x) Jpool[d.off_J + q] = J[q];
   const int w = tid;
   const bool live = w < d.walkers;
   int8_t* s = lat + static_cast<size_t>(w) * N;
@@ -105,22 +170,6 @@ __global__ void __launch_bounds__(1024) k_pre_batch(const PreDesc* __restrict__ 
   if (live) rng.init(key_u32(d.seed, static_cast<uint64_t>(d.sample)), 2 + static_cast<uint64_t>(w), 0);
   const double site_scale = (N - 1 + 0.999999);
   const uint32_t site_thr = static_cast<uint32_t>(N) * 2048u + 16384u;  // as MainDesc::site_thr
-  // u < exp(H[old] - H[new]) (wl.cu:536-537) for an integer count difference
-  // dd: always for dd >= 1 (exp(dd) > 1 >= u); never for dd <= -25
-  // (exp(dd) < 2^-33 <= u); else x < acc_thr[-dd], the least draw whose
-  // uniform reaches the device's exp(dd) (uniforms are monotone in the draw)
-  __shared__ uint32_t acc_thr[25];
-  if (tid < 25) {
-    const double e = exp(static_cast<double>(-tid));
-    unsigned long long lo = 0, hi = 1ull << 32;
-    while (lo < hi) {
-      const unsigned long long mid = (lo + hi) >> 1;
-      if (static_cast<double>(unit_float(static_cast<uint32_t>(mid))) >= e) hi = mid;
-      else lo = mid + 1;
-    }
-    acc_thr[tid] = static_cast<uint32_t>(lo);  // <= 2^32 - 128: u reaches 1 there
-  }
-  __syncthreads();
   bool ok = live;
   for (int it = 0; it < d.n_iter; ++it) {
     int hit = -1;
@@ -138,7 +187,7 @@ __global__ void __launch_bounds__(1024) k_pre_batch(const PreDesc* __restrict__ 
       const long long dd = static_cast<long long>(hist[io]) - static_cast<long long>(hist[in]);
       const uint32_t xa = rng.raw();
       const int ti = static_cast<int>(min(max(-dd, 0ll), 24ll));
-      acc = dd >= 1 || (dd >= -24 && xa < acc_thr[ti]);
+      acc = dd >= 1 || (dd >= -24 && xa < acc_thr[ti]);  // see fill_accept
       if (acc) s[m.site] = static_cast<int8_t>(-s[m.site]);
       energy = acc ? m.new_energy : energy;
       hit = acc ? in : io;
@@ -179,6 +228,26 @@ __global__ void __launch_bounds__(1024) k_pre_batch(const PreDesc* __restrict__ 
   }
 }
 
+// One CTA per problem.  CTAs of up to 256 threads may take 255 registers each:
+// the walk is latency-bound, and its loads are then issued further ahead.
+template <int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads, 1)
+  k_pre_batch(const PreDesc* __restrict__ descs, int n, int8_t* __restrict__ Jpool, uint8_t* __restrict__ seen_pool,
+              int8_t* __restrict__ found_pool, int* __restrict__ fflag_pool)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int p = blockIdx.x;
+  if (p >= n) return;
+  const PreDesc d = descs[p];
+  if (d.bonds == 0) {
+    pre_problem_i8(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
+  } else if (d.Y <= 16) {
+    pre_problem<false>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
+  } else {
+    pre_problem<true>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
+  }
+}
+
 }  // namespace
 
 // ------------------------------------------------------------ launchers ----
@@ -187,11 +256,12 @@ wlg_status launch_pre_batch(const PreDesc* d_descs, int n, int threads, int smem
                             int8_t* found_pool, int* fflag_pool, cudaStream_t s)
 {
   if (n == 0) return WLG_OK;
+  const auto kernel = threads <= 256 ? &k_pre_batch<256> : &k_pre_batch<1024>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_pre_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return WLG_ERR_CUDA;
   }
-  k_pre_batch<<<n, threads, smem, s>>>(d_descs, n, Jpool, seen_pool, found_pool, fflag_pool);
+  kernel<<<n, threads, smem, s>>>(d_descs, n, Jpool, seen_pool, found_pool, fflag_pool);
   return launch_status();
 }
 

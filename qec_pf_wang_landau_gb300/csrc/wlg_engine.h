@@ -35,7 +35,49 @@ struct PreDesc {
   long long off_found;  // int8 [n_int][N]
   long long off_fflag;  // int [n_int] flags, then int [n_int] energies
   int smem;             // dynamic shared memory of the CTA
+  int bonds;            // 1: the walk on bond words (wlg_pre.cuh), 0: on int8 lattices
 };
+
+// The walk on bond words takes rows of up to 32 sites, 32-bit counts and 22-bit
+// rounds.
+constexpr int kAcceptEntries = 27;
+WLG_HD inline int pre_hist_words(int len) { return (len + 4) & ~3; }  // one copy, a spare entry included
+WLG_HD inline bool pre_walk_fits(int X, int Y, int walkers, long long n_iter)
+{
+  return X >= 2 && Y >= 2 && Y <= 32 && walkers <= 1024 && n_iter * walkers < (1ll << 31) &&
+         n_iter < (1ll << 22) - 2;
+}
+
+// Shared memory of a walk on bond words (bytes; 16-byte aligned pieces).
+struct PreLayout {
+  int off_hist, off_claim, off_foundE, off_thr, off_col, off_row, off_J, off_base, off_words, bytes;
+};
+WLG_HD inline PreLayout pre_layout(int X, int Y, int len_hist, int n_int, int threads)
+{
+  auto up = [](long long x) { return static_cast<int>((x + 15) & ~15ll); };
+  PreLayout l{};
+  int o = 0;
+  l.off_hist = o;
+  o = up(o + 8ll * pre_hist_words(len_hist));
+  l.off_claim = o;
+  o = up(o + 4ll * n_int);
+  l.off_foundE = o;
+  o = up(o + 4ll * n_int);
+  l.off_thr = o;
+  o = up(o + 4ll * kAcceptEntries);
+  l.off_col = o;
+  o = up(o + 8ll * Y);
+  l.off_row = o;
+  o = up(o + 16ll * X);
+  l.off_J = o;  // coupling bits: right, then down
+  o = up(o + 8ll * X);
+  l.off_base = o;  // the start lattice's spin bits
+  o = up(o + 4ll * X);
+  l.off_words = o;
+  o = up(o + 4ll * X * (Y > 16 ? 2 : 1) * threads);
+  l.bytes = o;
+  return l;
+}
 
 // ----------------------------------------------------------- main run -----
 // Bit-packed lattices and couplings.  Lattices of more than 64 sites whose

@@ -367,6 +367,7 @@ wlg_status prerun_descs(const wlg_problem* probs, int n, wlg_result* results, Pr
   long long oJ = 0, oS = 0, oF = 0, oG = 0;
   threads = 32;
   smem = 0;
+  bool too_large = false;
   for (int p = 0; p < n; ++p) {
     if (check_problem(probs[p]) != WLG_OK) {
       err = "invalid problem " + std::to_string(p);
@@ -406,7 +407,12 @@ wlg_status prerun_descs(const wlg_problem* probs, int n, wlg_result* results, Pr
     oS += 4 * d.N + 1;
     oF += static_cast<long long>(d.n_int) * d.N;
     oG += 2 * d.n_int;
+    // a problem is taken when its walk on int8 lattices would fit
     d.smem = wlg::align16(8 * (4 * d.N + 1) + 8 * d.n_int + 16 + 2 * d.N + d.walkers * d.N);
+    if (d.smem > 227 * 1024) too_large = true;
+    const int bond_bytes = wlg::pre_layout(d.X, d.Y, 4 * d.N + 1, d.n_int, round32(d.walkers)).bytes;
+    d.bonds = wlg::pre_walk_fits(d.X, d.Y, d.walkers, d.n_iter) && bond_bytes <= 227 * 1024 ? 1 : 0;
+    if (d.bonds != 0) d.smem = bond_bytes;
     smem = std::max(smem, d.smem);
     threads = std::max(threads, round32(d.walkers));
     results[p].pre_flips = static_cast<long long>(q.pre_walkers) * q.pre_iterations;
@@ -415,7 +421,7 @@ wlg_status prerun_descs(const wlg_problem* probs, int n, wlg_result* results, Pr
   po.seen.assign(static_cast<size_t>(oS), 0);
   po.found.assign(static_cast<size_t>(oF), 0);
   po.fflag.assign(static_cast<size_t>(oG), 0);
-  if (smem > 227 * 1024) {
+  if (too_large) {
     err = "pre-run walkers x lattice too large for shared memory";
     return WLG_ERR_INVALID;
   }

@@ -18,6 +18,7 @@
 #include "../../include/wlg.h"
 #include "wlg_internal.h"
 #include "wlg_lattice.cuh"
+#include "wlg_pre.cuh"
 #include "wlg_rng.cuh"
 
 namespace wlg {
@@ -81,19 +82,120 @@ __global__ void k_calc_energy(int boundary, int* __restrict__ E, const int8_t* _
 }
 
 // --------------------------------------------------------------- pre-run ----
-// One CTA per sample, one thread per walker, the sample's histogram and
-// coarse-bin claims in shared memory.  Round-synchronous: decisions of round
-// r read the histogram after round r-1; barrier; increments and claims;
-// barrier; the lowest claimant of a still-empty bin stores its lattice.
-__global__ void k_prerun(int* __restrict__ E, int* __restrict__ flag_found, int8_t* __restrict__ lat,
-                         int8_t* __restrict__ found_lat, unsigned long long* __restrict__ H,
-                         uint64_t* __restrict__ seed_off, const int8_t* __restrict__ J,
-                         const int* __restrict__ off_lat, int E_min, int E_max, int n_iter, int X, int Y, int seed,
-                         unsigned n_int, int len_int, int wpi, int boundary)
+// One CTA per sample, one thread per walker (round-synchronous, see
+// wlg_pre.cuh).
+struct PrerunArgs {
+  int* E;
+  int* flag_found;
+  int8_t* lat;
+  int8_t* found_lat;
+  unsigned long long* H;
+  uint64_t* seed_off;
+  const int8_t* J;
+  const int* off_lat;
+  int E_min, E_max, n_iter, X, Y, seed, n_int, len_int, wpi, boundary;
+  int bonds;  // the walk on bond words fits
+};
+
+// The walk on bond words, on the caller's lattices, histogram and draws.
+template <bool kTwo>
+__device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char* smem)
 {
-  extern __shared__ unsigned long long sm[];
+  constexpr int kW = kTwo ? 2 : 1;
+  const int k = blockIdx.x, w = threadIdx.x, X = a.X, Y = a.Y, N = X * Y;
+  const int threads = blockDim.x, len = a.E_max - a.E_min + 1, Lh = pre_hist_words(len);
+  const bool live = w < a.wpi;
+  const size_t t = static_cast<size_t>(k) * a.wpi + w;
+  const PreLayout l = pre_layout(X, Y, len, a.n_int, threads);
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + l.off_hist);
+  uint32_t* thr = reinterpret_cast<uint32_t*>(smem + l.off_thr);
+  uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
+  uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
+  uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
+  const PreWalk p{X, Y, a.boundary, a.E_min, a.E_max, a.n_int, min(a.len_int, 1 << 15), a.n_iter, threads, hist,
+                  reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr, col,
+                  row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words),
+                  a.found_lat + static_cast<long long>(k) * a.n_int * N};
+  const PreSync sync{threads};
+  for (int q = w; q < Lh; q += threads) {
+    const uint32_t h = q < len ? static_cast<uint32_t>(a.H[static_cast<size_t>(k) * len + q]) : 0u;
+    hist[q] = hist[Lh + q] = h;
+  }
+  for (int q = w; q < a.n_int; q += threads)
+    p.claim[q] = a.flag_found[static_cast<size_t>(k) * a.n_int + q] == 0 ? kPreEmpty : 0u;
+  for (int q = w; q < X; q += threads) {
+    const int8_t* Jk = a.J + static_cast<size_t>(k) * 2 * N + q * Y;
+    uint32_t r = 0, dn = 0;
+    for (int j = 0; j < Y; ++j) {
+      r |= Jk[j] < 0 ? 1u << j : 0u;
+      dn |= Jk[N + j] < 0 ? 1u << j : 0u;
+    }
+    Jr[q] = r;
+    Jr[X + q] = dn;
+  }
+  fill_accept(thr, w);
+  fill_bonds<kTwo>(col, row, X, Y, a.boundary, w, threads);
+  sync();
+  int8_t* s = live ? a.lat + a.off_lat[t] : nullptr;
+  auto row_bits = [&](int i) {
+    uint32_t r = 0;
+    for (int j = 0; j < Y; ++j) r |= s[i * Y + j] < 0 ? 1u << j : 0u;
+    return r;
+  };
+  uint32_t s0 = 0;
+  int E = 0;
+  uint64_t pos = 0;
+  if (live) {
+    const uint32_t first = row_bits(0);
+    uint32_t r = first;
+    for (int i = 0; i < X; ++i) {
+      const uint32_t dn = i + 1 < X ? row_bits(i + 1) : first;
+      uint32_t h, v = 0;
+      bond_words<kTwo>(r, dn, Jr[i], Jr[X + i], Y, a.boundary != 0, i + 1 == X, h, v);
+      p.words[i * kW * threads + w] = h;
+      if constexpr (kTwo) p.words[(i * kW + 1) * threads + w] = v;
+      r = dn;
+    }
+    s0 = first & 1u;
+    E = a.E[t];
+    pos = a.seed_off[t];
+  } else {
+    for (int q = 0; q < X * kW; ++q) p.words[q * threads + w] = 0;
+  }
+  pre_walk<kTwo, true>(p, sync, w, live, key_u32(a.seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), pos, E,
+                       s0);
+  for (int q = w; q < len; q += threads) a.H[static_cast<size_t>(k) * len + q] = hist[q];
+  for (int q = w; q < a.n_int; q += threads)
+    if (p.claim[q] != kPreEmpty && p.claim[q] != 0u) a.flag_found[static_cast<size_t>(k) * a.n_int + q] = 1;
+  if (live) {
+    // spins from the bonds: down column 0, then along each row
+    uint32_t edge = s0;
+    for (int i = 0; i < X; ++i) {
+      const uint32_t word = p.words[i * kW * threads + w];
+      const uint32_t turn = word ^ Jr[i];
+      uint32_t sp = edge;
+      for (int j = 0; j < Y; ++j) {
+        s[i * Y + j] = sp != 0 ? -1 : 1;
+        sp ^= (turn >> j) & 1u;
+      }
+      edge ^= ((kTwo ? p.words[(i * kW + 1) * threads + w] : word >> 16) ^ Jr[X + i]) & 1u;
+    }
+    a.E[t] = E;
+    a.seed_off[t] = pos;
+  }
+}
+
+// The walk on the caller's int8 lattices with 64-bit counts, for everything
+// else: values other than +-1, odd draw offsets, counts of 2^31 and more, rows of
+// more than 32 sites.
+__device__ __forceinline__ void prerun_i8(const PrerunArgs& a, unsigned char* smem)
+{
+  int* const E = a.E;
+  int* const flag_found = a.flag_found;
+  unsigned long long* const H = a.H;
+  const int E_min = a.E_min, E_max = a.E_max, X = a.X, Y = a.Y, n_int = a.n_int, wpi = a.wpi, boundary = a.boundary;
   const int len_hist = E_max - E_min + 1;
-  unsigned long long* hist = sm;
+  unsigned long long* hist = reinterpret_cast<unsigned long long*>(smem);
   int* claim = reinterpret_cast<int*>(hist + len_hist);
   int* found = claim + n_int;
 
@@ -104,7 +206,7 @@ __global__ void k_prerun(int* __restrict__ E, int* __restrict__ flag_found, int8
   const size_t t = static_cast<size_t>(k) * wpi + w;
 
   for (int q = threadIdx.x; q < len_hist; q += blockDim.x) hist[q] = H[static_cast<size_t>(k) * len_hist + q];
-  for (int q = threadIdx.x; q < static_cast<int>(n_int); q += blockDim.x) {
+  for (int q = threadIdx.x; q < n_int; q += blockDim.x) {
     claim[q] = INT_MAX;
     found[q] = flag_found[static_cast<size_t>(k) * n_int + q];
   }
@@ -114,16 +216,16 @@ __global__ void k_prerun(int* __restrict__ E, int* __restrict__ flag_found, int8
   int8_t* s = nullptr;
   bool ok = true;
   if (live) {
-    rng.init(key_u32(seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), seed_off[t]);
+    rng.init(key_u32(a.seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), a.seed_off[t]);
     energy = E[t];
-    s = lat + off_lat[t];
+    s = a.lat + a.off_lat[t];
     ok = energy >= E_min && energy <= E_max;  // a walker outside the range never indexes the histogram
   }
-  const int8_t* Jk = J + static_cast<size_t>(k) * 2 * N;
+  const int8_t* Jk = a.J + static_cast<size_t>(k) * 2 * N;
   const double site_scale = (N - 1 + 0.999999);
   __syncthreads();
 
-  for (int it = 0; it < n_iter; ++it) {
+  for (int it = 0; it < a.n_iter; ++it) {
     int hit = -1;
     bool acc = false;
     if (live && ok) {
@@ -150,25 +252,54 @@ __global__ void k_prerun(int* __restrict__ E, int* __restrict__ flag_found, int8
     int bin = -1;
     if (hit >= 0) atomicAdd(&hist[hit], 1ull);
     if (acc) {
-      const int q = (energy - E_min) / len_int;
-      bin = (q < static_cast<int>(n_int)) ? q : static_cast<int>(n_int) - 1;
+      const int q = (energy - E_min) / a.len_int;
+      bin = (q < n_int) ? q : n_int - 1;
       if (found[bin] == 0) atomicMin(&claim[bin], w);
       else bin = -1;
     }
     __syncthreads();
     if (bin >= 0 && claim[bin] == w && found[bin] == 0) {
       found[bin] = 1;
-      int8_t* dst = found_lat + (static_cast<size_t>(k) * n_int + bin) * N;
+      int8_t* dst = a.found_lat + (static_cast<size_t>(k) * n_int + bin) * N;
       for (int q = 0; q < N; ++q) dst[q] = s[q];
     }
   }
   __syncthreads();
   for (int q = threadIdx.x; q < len_hist; q += blockDim.x) H[static_cast<size_t>(k) * len_hist + q] = hist[q];
-  for (int q = threadIdx.x; q < static_cast<int>(n_int); q += blockDim.x)
+  for (int q = threadIdx.x; q < n_int; q += blockDim.x)
     flag_found[static_cast<size_t>(k) * n_int + q] = found[q];
   if (live) {
     E[t] = energy;
-    seed_off[t] = rng.pos;
+    a.seed_off[t] = rng.pos;
+  }
+}
+
+template <int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int k = blockIdx.x, N = a.X * a.Y, len = a.E_max - a.E_min + 1;
+  bool fast = a.bonds != 0;
+  if (fast) {
+    for (int q = threadIdx.x; q < 2 * N; q += blockDim.x) {
+      const int8_t v = a.J[static_cast<size_t>(k) * 2 * N + q];
+      fast = fast && (v == 1 || v == -1);
+    }
+    const unsigned long long most = (1ull << 31) - 1 - static_cast<unsigned long long>(a.n_iter) * a.wpi;
+    for (int q = threadIdx.x; q < len; q += blockDim.x) fast = fast && a.H[static_cast<size_t>(k) * len + q] <= most;
+    if (static_cast<int>(threadIdx.x) < a.wpi) {
+      const size_t t = static_cast<size_t>(k) * a.wpi + threadIdx.x;
+      const int8_t* s = a.lat + a.off_lat[t];
+      for (int q = 0; q < N; ++q) fast = fast && (s[q] == 1 || s[q] == -1);
+      fast = fast && (a.seed_off[t] & 1u) == 0;
+    }
+  }
+  if (__syncthreads_and(fast ? 1 : 0) == 0) {
+    prerun_i8(a, smem);
+  } else if (a.Y <= 16) {
+    prerun_bonds<false>(a, smem);
+  } else {
+    prerun_bonds<true>(a, smem);
   }
 }
 
@@ -475,18 +606,26 @@ wlg_status wlg_wang_landau_pre_run(int* d_energy, int* d_flag_found_interval, in
   const int R = static_cast<int>(num_total_walker / walker_per_sample);
   if (R == 0 || num_iterations <= 0) return WLG_OK;
   const int len_hist = E_max - E_min + 1;
-  const size_t smem = static_cast<size_t>(len_hist) * sizeof(unsigned long long) + 2 * sizeof(int) * num_intervals;
+  size_t smem = static_cast<size_t>(len_hist) * sizeof(unsigned long long) + 2 * sizeof(int) * num_intervals;
   if (smem > 200 * 1024) return WLG_ERR_INVALID;
+  const int threads = (walker_per_sample + 31) / 32 * 32;
+  PrerunArgs a{d_energy, d_flag_found_interval, d_lattice, d_found_interval_lattice, d_histogram, d_seed_offset, d_J,
+               d_offset_lattice, E_min, E_max, num_iterations, X, Y, seed, static_cast<int>(num_intervals), len_interval,
+               walker_per_sample, boundary, 0};
+  if (static_cast<long long>(X) * Y <= 4096 && pre_walk_fits(X, Y, walker_per_sample, num_iterations)) {
+    const size_t bytes = static_cast<size_t>(pre_layout(X, Y, len_hist, a.n_int, threads).bytes);
+    if (bytes <= 227 * 1024) {
+      a.bonds = 1;
+      smem = std::max(smem, bytes);
+    }
+  }
   cudaStream_t s = as_stream(stream);
+  const auto kernel = threads <= 256 ? &k_prerun<256> : &k_prerun<1024>;
   if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(k_prerun, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
       return WLG_ERR_CUDA;
   }
-  const int threads = (walker_per_sample + 31) / 32 * 32;
-  k_prerun<<<R, threads, smem, s>>>(d_energy, d_flag_found_interval, d_lattice, d_found_interval_lattice, d_histogram,
-                                    d_seed_offset, d_J, d_offset_lattice, E_min, E_max, num_iterations, X, Y, seed,
-                                    num_intervals, len_interval, walker_per_sample, boundary);
+  kernel<<<R, threads, smem, s>>>(a);
   return launch_status();
 }
 
