@@ -19,6 +19,7 @@
 #include "wlg_internal.h"
 #include "wlg_lattice.cuh"
 #include "wlg_pre.cuh"
+#include "wlg_sweep.cuh"
 #include "wlg_rng.cuh"
 
 namespace wlg {
@@ -304,45 +305,53 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
 }
 
 // ------------------------------------------------------- main WL sweep -----
-// wl.cu:1033-1175, one thread per walker.
-__global__ void k_wang_landau(int8_t* __restrict__ lat, const int8_t* __restrict__ J,
-                              unsigned long long* __restrict__ H, double* __restrict__ logG,
-                              const double* __restrict__ factor, int* __restrict__ E, int* __restrict__ newE,
-                              uint64_t* __restrict__ off_iter, int* __restrict__ found, const int* __restrict__ start,
-                              const int* __restrict__ end, const int* __restrict__ off_hist,
-                              const int* __restrict__ off_lat, const int8_t* __restrict__ cond,
-                              const int8_t* __restrict__ spectrum, const int* __restrict__ off_spec,
-                              const int* __restrict__ cond_inter, int X, int Y, int n_iter, int num_lattices,
-                              int n_int, int wpi, int seed, int boundary)
+// wl.cu:1033-1175 on the caller's arrays.
+struct SweepArgs {
+  int8_t* lat;
+  const int8_t* J;
+  unsigned long long* H;
+  double* logG;
+  const double* factor;
+  int* E;
+  int* newE;
+  uint64_t* off_iter;
+  int* found;
+  const int *start, *end, *off_hist, *off_lat;
+  const int8_t *cond, *spectrum;
+  const int *off_spec, *cond_inter;
+  int X, Y, n_iter, num_lattices, n_int, wpi, seed, boundary;
+  int L;           // bins a walker's column holds (k_wl_sweep)
+  uint32_t magic;  // site / Y = site * magic >> 20
+};
+
+// One walker by one thread, straight on global memory.
+__device__ __forceinline__ void sweep_global(const SweepArgs& a, int t)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= num_lattices) return;
-  const int W = wpi / n_int;
-  const int k = t / wpi;
+  const int W = a.wpi / a.n_int;
+  const int k = t / a.wpi;
   const int b = t / W;
-  if (cond_inter[k] == -1) return;
-  const int N = X * Y;
+  const int N = a.X * a.Y;
   Stream rng;
-  rng.init(key_u32(seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t % wpi), off_iter[t]);
-  int8_t* s = lat + off_lat[t];
-  const int8_t* Jk = J + static_cast<size_t>(k) * 2 * N;
-  const int8_t* mask = spectrum + off_spec[k] - start[k * n_int];
-  const int e_first = start[k * n_int], e_last = end[k * n_int + n_int - 1];
-  const int lo = start[b], hi = end[b];
-  unsigned long long* Hw = H + off_hist[t] - lo;
-  double* Gw = logG + off_hist[t] - lo;
-  const double lnf = log(factor[t]);
+  rng.init(key_u32(a.seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t % a.wpi), a.off_iter[t]);
+  int8_t* s = a.lat + a.off_lat[t];
+  const int8_t* Jk = a.J + static_cast<size_t>(k) * 2 * N;
+  const int8_t* mask = a.spectrum + a.off_spec[k] - a.start[k * a.n_int];
+  const int e_first = a.start[k * a.n_int], e_last = a.end[k * a.n_int + a.n_int - 1];
+  const int lo = a.start[b], hi = a.end[b];
+  unsigned long long* Hw = a.H + a.off_hist[t] - lo;
+  double* Gw = a.logG + a.off_hist[t] - lo;
+  const double lnf = log(a.factor[t]);
   const double site_scale = (N - 1 + 0.999999);
-  const bool frozen = cond[b] != 0;
-  int energy = E[t];
+  const bool frozen = a.cond[b] != 0;
+  int energy = a.E[t];
   int flag = 0;
-  for (int it = 0; it < n_iter; ++it) {
-    const Move m = propose_i8(rng, s, Jk, energy, X, Y, site_scale, boundary);
+  for (int it = 0; it < a.n_iter; ++it) {
+    const Move m = propose_i8(rng, s, Jk, energy, a.X, a.Y, site_scale, a.boundary);
     // wl.cu:1091-1104; an energy outside the sample's spectrum range counts
     // as new too (the reference reads the mask out of bounds there).
     if (m.new_energy < e_first || m.new_energy > e_last || mask[m.new_energy] != 1) {
       flag = t + 1;
-      newE[t] = m.new_energy;
+      a.newE[t] = m.new_energy;
       break;
     }
     const bool inside = m.new_energy <= hi && m.new_energy >= lo;
@@ -369,9 +378,189 @@ __global__ void k_wang_landau(int8_t* __restrict__ lat, const int8_t* __restrict
       }
     }
   }
-  if (n_iter > 0) found[t] = flag;
-  E[t] = energy;
-  off_iter[t] = rng.pos;
+  if (a.n_iter > 0) a.found[t] = flag;
+  a.E[t] = energy;
+  a.off_iter[t] = rng.pos;
+}
+
+__global__ void k_wang_landau(const SweepArgs a)
+{
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= a.num_lattices || a.cond_inter[t / a.wpi] == -1) return;
+  sweep_global(a, t);
+}
+
+// Shared memory of k_wl_sweep: one warp of 32 walkers (bytes).
+struct SweepLayout {
+  int off_desc, off_J, off_tab, off_ring, off_lat, off_pair, bytes;
+};
+WLG_HD inline SweepLayout sweep_layout(int X, int Y, int L, int lg)
+{
+  SweepLayout l{};
+  int o = 0;
+  l.off_desc = o;
+  o = align16(o + static_cast<int>(sizeof(MainDesc)));
+  l.off_J = o;
+  o = align16(o + 8 * X);
+  l.off_tab = o;
+  o = align16(o + align16(8 * Y) + 16 * X);
+  l.off_ring = o;
+  o = align16(o + kRingWarpBytes);
+  l.off_lat = o;
+  o = align16(o + 4 * X * 32);
+  l.off_pair = o;
+  o = align16(o + 8 * (L + 2 * guard_bins(lg)) * 32);
+  l.bytes = o;
+  return l;
+}
+
+// The sweep of the persistent main run (wlg_sweep.cuh) on the caller's arrays:
+// one warp takes 32 walkers of a sample, packs their lattices (bonds or rows)
+// and the bins of their windows into shared memory, and writes lattices,
+// visits and log g back at the end.  The step on global memory is one chain of
+// dependent loads and an FP64 exp, about 2.6 us; here 0.13 us, and packing and
+// unpacking cost some 10 us a call.  GB300, 1024 walkers on 10x10, 200 steps:
+// see wlg_wang_landau.  Warps with arrays the sweep does not take (couplings
+// or spins other than +-1, log g of 2^100 and more, factors below 1, an energy
+// outside its window, windows wider than the columns) walk on global memory.
+template <int kStore>
+__global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
+{
+  constexpr bool kBonds = kStore == kStoreBonds;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int groups = (a.wpi + 31) / 32, lane = threadIdx.x;
+  const int k = blockIdx.x / groups, w = (blockIdx.x - k * groups) * 32 + lane, t = k * a.wpi + w;
+  const bool live = w < a.wpi && t < a.num_lattices;
+  if (a.cond_inter[k] == -1) return;
+  const int X = a.X, Y = a.Y, N = X * Y, lg = a.boundary == 0 ? 2 : 1, guard = guard_bins(lg);
+  const bool open = a.boundary != 0;
+  const SweepLayout l = sweep_layout(X, Y, a.L, lg);
+  MainDesc& d = *reinterpret_cast<MainDesc*>(smem + l.off_desc);
+  uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
+  uint32_t* words = reinterpret_cast<uint32_t*>(smem + l.off_lat) + lane;
+  float2* pair = reinterpret_cast<float2*>(smem + l.off_pair) + guard * 32 + lane;
+  if (lane == 0) {
+    d.X = X;
+    d.Y = Y;
+    d.N = N;
+    d.boundary = a.boundary;
+    d.lg = lg;
+    d.site_thr = static_cast<uint32_t>(N) * 2048u + 16384u;
+    d.site_scale = (N - 1 + 0.999999);
+    d.site_magic = a.magic;
+  }
+  bool ok = true;
+  const int8_t* Jk = a.J + static_cast<size_t>(k) * 2 * N;
+  for (int q = lane; q < 2 * X; q += 32) {  // coupling bits: right, then down
+    const int8_t* src = Jk + q * Y;
+    uint32_t bits = 0;
+    for (int j = 0; j < Y; ++j) {
+      ok = ok && (src[j] == 1 || src[j] == -1);
+      bits |= src[j] < 0 ? 1u << j : 0u;
+    }
+    Jr[q] = bits;
+  }
+  uint2* col = reinterpret_cast<uint2*>(smem + l.off_tab);
+  fill_bond_tables(col, reinterpret_cast<uint4*>(smem + l.off_tab + align16(8 * Y)), X, Y, open, 2 * (256 >> lg), lane, 32);
+  __syncwarp();
+  const int b = t / (a.wpi / a.n_int);
+  const int e_first = a.start[k * a.n_int], e_last = a.end[k * a.n_int + a.n_int - 1];
+  const int8_t* mask = a.spectrum + a.off_spec[k] - e_first;
+  auto is_bad = [&](int En) { return En < e_first || En > e_last || mask[En] != 1; };
+  Walker<false> wk;
+  wk.s0 = 0;
+  wk.lo = wk.hi = wk.bb = wk.len = wk.E = 0;
+  int8_t* s = nullptr;
+  double lnf = 0.0;
+  unsigned long long* H = nullptr;
+  double* G = nullptr;
+  if (live) {
+    s = a.lat + a.off_lat[t];
+    auto row_bits = [&](int i) {
+      uint32_t r = 0;
+      for (int j = 0; j < Y; ++j) {
+        const int8_t v = s[i * Y + j];
+        ok = ok && (v == 1 || v == -1);
+        r |= v < 0 ? 1u << j : 0u;
+      }
+      return r;
+    };
+    const uint32_t first = row_bits(0);
+    uint32_t r = first;
+    for (int i = 0; i < X; ++i) {
+      const uint32_t below = i + 1 < X ? row_bits(i + 1) : first;
+      words[i * 32] = kBonds ? bond_word(r, below, Jr[i], Jr[X + i], Y, open, i + 1 == X) : r;
+      r = below;
+    }
+    wk.s0 = first & 1u;
+    wk.E = a.E[t];
+    wk.lo = a.start[b];
+    wk.hi = a.end[b];
+    ok = ok && wk.E >= wk.lo && wk.E <= wk.hi;
+    wk.bb = wk.lo + ((wk.E - wk.lo) & ((1 << lg) - 1));  // the walker's energies, a step apart
+    wk.len = ((wk.hi - wk.bb) >> lg) + 1;
+    ok = ok && wk.len <= a.L;
+    lnf = log(a.factor[t]);
+    ok = ok && lnf >= 0.0 && lnf < 1e6;
+    H = a.H + a.off_hist[t] + (wk.bb - wk.lo);
+    G = a.logG + a.off_hist[t] + (wk.bb - wk.lo);
+    if (ok)
+      for (int c = 0; c < wk.len; ++c) ok = ok && (__double2hiint(G[c << lg]) & 0x7FFFFFFF) < 0x46300000;  // |g| < 2^100
+  }
+  if (__any_sync(0xFFFFFFFFu, !ok)) {
+    if (live) sweep_global(a, t);
+    return;
+  }
+  const unsigned wmask = __ballot_sync(0xFFFFFFFFu, live);
+  if (!live) return;
+  for (int c = -guard; c < wk.len + guard; ++c) {
+    const int En = wk.bb + c * (1 << lg);
+    pair[c * 32] = make_float2(is_bad(En) ? __int_as_float(0x7FC00000)
+                                          : (En >= wk.lo && En <= wk.hi ? 0.0f : __int_as_float(0x7F800000)),
+                               0.0f);
+  }
+  wk.lt.r = 0;
+  wk.lt.a = shared_addr(words);
+  wk.lt.stride = 128u;
+  wk.pair = pair;
+  wk.ring_a = shared_addr(smem + l.off_ring) + 4 * lane;
+  wk.rng.init(key_u32(a.seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(w), a.off_iter[t]);
+  wk.start();
+  const uint32_t tab_a = shared_addr(col);
+  const SweepTeam team{d, 32, tab_a, tab_a + align16(8 * Y), Jr, Jr + X, 0, 0};
+  const bool frozen = a.cond[b] != 0;
+  int flag = 0;
+  auto log_g = [&](int c) { return G[c << lg]; };
+  auto new_energy = [&](int En, int) {
+    flag = t + 1;
+    a.newE[t] = En;
+  };
+  auto fold = [&](float, int, bool) {
+    wk.fresh = false;
+    if (frozen) return;
+    for (int c = 0; c < wk.len; ++c) {
+      const uint32_t n = static_cast<uint32_t>(pair[c * 32].y);
+      if (n == 0) continue;
+      pair[c * 32].y = 0.0f;
+      H[c << lg] += n;
+      G[c << lg] = add_times<true>(G[c << lg], lnf, n);
+    }
+  };
+  wl_sweep<kStore, false, true>(team, wk, wmask, a.n_iter, frozen, lnf, log_g, is_bad, new_energy, fold);
+  // lattices: rows as they are; bonds down column 0, then along each row
+  uint32_t edge = wk.s0;
+  for (int i = 0; i < X; ++i) {
+    const uint32_t word = words[i * 32], turn = word ^ Jr[i];
+    uint32_t sp = edge;
+    for (int j = 0; j < Y; ++j) {
+      s[i * Y + j] = (kBonds ? sp : (word >> j) & 1u) != 0 ? -1 : 1;
+      sp ^= (turn >> j) & 1u;
+    }
+    edge ^= ((word >> 16) ^ Jr[X + i]) & 1u;
+  }
+  a.found[t] = flag;
+  a.E[t] = wk.E;
+  a.off_iter[t] = wk.rng.pos;
 }
 
 // -------------------------------------------------------------- flatness ----
@@ -641,10 +830,34 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
       walker_per_sample % num_intervals != 0 || num_lattices < 0)
     return WLG_ERR_INVALID;
   if (num_lattices == 0) return WLG_OK;
-  k_wang_landau<<<blocks_for(static_cast<size_t>(num_lattices)), kThreads, 0, as_stream(stream)>>>(
-    d_lattice, d_J, d_H, d_logG, d_factor, d_energy, d_new_energy, d_offset_iter, d_found, d_start, d_end,
-    d_offset_histogram, d_offset_lattice, d_cond, d_spectrum, d_offset_spectrum, d_cond_sample, X, Y, num_iterations,
-    num_lattices, num_intervals, walker_per_sample, seed, boundary);
+  SweepArgs a{d_lattice, d_J, d_H, d_logG, d_factor, d_energy, d_new_energy, d_offset_iter, d_found, d_start, d_end,
+              d_offset_histogram, d_offset_lattice, d_cond, d_spectrum, d_offset_spectrum, d_cond_sample, X, Y,
+              num_iterations, num_lattices, num_intervals, walker_per_sample, seed, boundary, 0, 0};
+  cudaStream_t s = as_stream(stream);
+  const int N = X * Y, lg = boundary == 0 ? 2 : 1;
+  bool packed = X >= 2 && Y >= 2 && Y <= 32 && static_cast<long long>(X) * Y <= 4096 && num_iterations > 0;
+  if (packed) {
+    // Columns for windows of up to 8 / num_intervals of the energy range: the
+    // last window is up to twice as long as the others, which take
+    // 1 / (1 + overlap (num_intervals - 1)) of it.
+    const int full = (4 * N >> lg) + 1;
+    a.L = std::min(full, 8 * full / num_intervals + 8);
+    a.magic = static_cast<uint32_t>(((1u << 20) + Y - 1) / Y);
+    for (int site = 0; site < N; ++site)
+      packed = packed && static_cast<int>((static_cast<uint32_t>(site) * a.magic) >> 20) == site / Y;
+    packed = packed && sweep_layout(X, Y, a.L, lg).bytes <= 227 * 1024;
+  }
+  if (!packed) {
+    k_wang_landau<<<blocks_for(static_cast<size_t>(num_lattices)), kThreads, 0, s>>>(a);
+    return launch_status();
+  }
+  const int smem = sweep_layout(X, Y, a.L, lg).bytes;
+  const auto kernel = Y <= 16 ? &k_wl_sweep<kStoreBonds> : &k_wl_sweep<kStoreRows>;
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return WLG_ERR_CUDA;
+  const int samples = (num_lattices + walker_per_sample - 1) / walker_per_sample;
+  kernel<<<samples * ((walker_per_sample + 31) / 32), 32, smem, s>>>(a);
   return launch_status();
 }
 

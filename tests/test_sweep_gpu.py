@@ -1,0 +1,51 @@
+"""The sweep operator against the oracle, array by array, at the edges of its
+dispatch: warps with 1 to 32 walkers, rows of 16, 17 and 33 sites, one step, a
+sweep longer than a part, log g from zero and far along, finished windows, and
+arrays that only the walk on global memory takes."""
+import numpy as np
+import pytest
+
+from tests.helpers import Dev, assert_state_equal, copy_state, mainrun_state, o_wang_landau, prerun_outputs
+
+pytestmark = pytest.mark.gpu
+
+#  X, Y, boundary, R, I, W, overlap, prob, n_iter, sweeps, option
+SWEEPS = [
+    (4, 4, 0, 1, 1, 1, 0.25, 0.04, 300, 3, ""), (6, 6, 0, 2, 11, 3, 0.25, 0.08, 200, 3, ""),
+    (6, 6, 1, 2, 8, 4, 0.25, 0.08, 1, 5, ""), (5, 16, 0, 2, 5, 7, 0.25, 0.10, 333, 3, ""),
+    (5, 17, 1, 2, 5, 7, 0.25, 0.10, 333, 3, ""), (3, 32, 0, 1, 6, 6, 0.25, 0.10, 200, 3, ""),
+    (3, 33, 0, 1, 6, 6, 0.25, 0.10, 200, 2, ""), (9, 9, 0, 1, 16, 8, 0.25, 0.10, 500, 3, "far"),
+    (9, 9, 1, 2, 12, 5, 0.25, 0.10, 500, 3, "far"), (2, 2, 1, 1, 1, 40, 0.25, 0.0, 100, 3, ""),
+    (6, 6, 0, 1, 40, 2, 0.05, 0.08, 200, 2, "narrow overlap"), (4, 4, 0, 1, 2, 2, 0.25, 0.04, 70001, 1, ""),
+    (6, 6, 0, 1, 8, 4, 0.25, 0.08, 200, 2, "negative"), (6, 6, 0, 1, 8, 4, 0.25, 0.08, 200, 2, "factor"),
+    (6, 6, 1, 2, 8, 5, 0.25, 0.08, 200, 2, "diluted"), (6, 6, 0, 2, 8, 5, 0.25, 0.08, 300, 2, "missed"),
+]
+
+
+@pytest.mark.parametrize("X,Y,boundary,R,I,W,overlap,prob,n_iter,sweeps,option", SWEEPS)
+def test_sweep_operator_edges(cuda, X, Y, boundary, R, I, W, overlap, prob, n_iter, sweeps, option):
+    seed = 12345
+    pre = prerun_outputs(X, Y, boundary, prob, "i", seed, R, 128, min(48, X * Y), 100 * X * Y)
+    st = mainrun_state(pre, I, W, overlap)
+    rng = np.random.default_rng(3)
+    T = R * I * W
+    if option == "far":  # a run in progress: log g in the hundreds, small factors, every third window finished
+        st["logG"][:] = 300.0 + 40.0 * rng.random(len(st["logG"]))
+        st["H"][:] = rng.integers(0, 1 << 40, len(st["H"])).astype(np.uint64)
+        st["factor"][:] = np.exp(2.0 ** -np.repeat(rng.integers(1, 40, R * I), W).astype(np.float64))
+        st["cond"][::3] = 1
+    if option == "negative":
+        st["logG"][:] = -5.0 * rng.random(len(st["logG"]))
+    if option == "factor":
+        st["factor"][::7] = 0.9
+    if option == "diluted":
+        st["J"][::5] = 0
+        st["spectrum"][:] = 1
+    if option == "missed":  # energies taken out of the spectrum: walkers stop there
+        on = np.nonzero(st["spectrum"])[0]
+        st["spectrum"][on[len(on) // 3::len(on) // 3]] = 0
+    dev = Dev(cuda, copy_state(st))
+    for it in range(sweeps):
+        o_wang_landau(st, n_iter, seed)
+        dev.wang_landau(n_iter, seed)
+        assert_state_equal(dev.snapshot(), st, f"sweep {it}")
