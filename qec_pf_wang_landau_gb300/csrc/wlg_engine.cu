@@ -58,7 +58,7 @@ __device__ __forceinline__ int8_t draw_spin(const PreDesc& d, int q)
 }
 
 // The whole pre-run of one problem on bond words.
-template <bool kTwo>
+template <bool kTwo, bool kKeys>
 __device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* smem, int8_t* __restrict__ Jpool,
                                             uint8_t* __restrict__ seen_pool, int8_t* __restrict__ found_pool,
                                             int* __restrict__ fflag_pool)
@@ -115,7 +115,7 @@ __device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* sme
   int E = 2 * static_cast<int>(unsat) - bonds;
   uint32_t s0 = base[0] & 1u;
   uint64_t pos = 0;
-  pre_walk<kTwo, false>(p, sync, w, w < d.walkers, key_u32(d.seed, static_cast<uint64_t>(d.sample)),
+  pre_walk<kTwo, false, kKeys>(p, sync, w, w < d.walkers, key_u32(d.seed, static_cast<uint64_t>(d.sample)),
                         2 + static_cast<uint64_t>(w), pos, E, s0);
   for (int q = tid; q < L; q += threads) seen_pool[d.off_seen + q] = hist[q] != 0 ? 1 : 0;
   for (int q = tid; q < d.n_int; q += threads) {
@@ -242,9 +242,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
   if (d.bonds == 0) {
     pre_problem_i8(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
   } else if (d.Y <= 16) {
-    pre_problem<false>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
+    pre_problem<false, kMaxThreads <= 256>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
   } else {
-    pre_problem<true>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
+    pre_problem<true, kMaxThreads <= 256>(d, smem, Jpool, seen_pool, found_pool, fflag_pool);
   }
 }
 

@@ -99,7 +99,7 @@ struct PrerunArgs {
 };
 
 // The walk on bond words, on the caller's lattices, histogram and draws.
-template <bool kTwo>
+template <bool kTwo, bool kKeys>
 __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char* smem)
 {
   constexpr int kW = kTwo ? 2 : 1;
@@ -163,7 +163,7 @@ __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char*
   } else {
     for (int q = 0; q < X * kW; ++q) p.words[q * threads + w] = 0;
   }
-  pre_walk<kTwo, true>(p, sync, w, live, key_u32(a.seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), pos, E,
+  pre_walk<kTwo, true, kKeys>(p, sync, w, live, key_u32(a.seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), pos, E,
                        s0);
   for (int q = w; q < len; q += threads) a.H[static_cast<size_t>(k) * len + q] = hist[q];
   for (int q = w; q < a.n_int; q += threads)
@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
   if (__syncthreads_and(fast ? 1 : 0) == 0) {
     prerun_i8(a, smem);
   } else if (a.Y <= 16) {
-    prerun_bonds<false>(a, smem);
+    prerun_bonds<false, kMaxThreads <= 256>(a, smem);
   } else {
-    prerun_bonds<true>(a, smem);
+    prerun_bonds<true, kMaxThreads <= 256>(a, smem);
   }
 }
 
@@ -419,9 +419,10 @@ WLG_HD inline SweepLayout sweep_layout(int X, int Y, int L, int lg)
 // and the bins of their windows into shared memory, and writes lattices,
 // visits and log g back at the end.  The step on global memory is one chain of
 // dependent loads and an FP64 exp, about 2.6 us; here 0.13 us, and packing and
-// unpacking cost some 10 us a call.  GB300, 1024 walkers on 10x10, 200 steps:
-// see wlg_wang_landau.  Warps with arrays the sweep does not take (couplings
-// or spins other than +-1, log g of 2^100 and more, factors below 1, an energy
+// unpacking cost some 10 us a call.  GB300: an outer iteration of 16 samples of
+// 10x10 on the operators (1024 walkers, 200 steps) 0.56 -> 0.047 ms, a whole run
+// of 16 samples of 6x6 on them 45 -> 5.5 ms.  Warps with arrays the sweep does
+// not take (couplings or spins other than +-1, log g of 2^100 and more, factors below 1, an energy
 // outside its window, windows wider than the columns) walk on global memory.
 template <int kStore>
 __global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)

@@ -24,10 +24,11 @@
 // them, and rare cases sit in one warp-uniform block so that nothing else
 // branches).  GB300, 128 walkers a sample, time per round, against int8 lattices
 // with 64-bit counts, an acceptance table read after the histogram and two
-// barriers: 24x24 1.09 -> 0.26 us, 16x16 1.12 -> 0.24 us; 152 samples of 16x16,
-// 25600 rounds, 28.6 -> 6.0 ms; the operator, 64 samples of 9x9, 1000 rounds,
-// with set-up 2.05 -> 0.36 ms.  (The same words with branches around site
-// fallback and claims: 0.40 us.)
+// barriers: 24x24 1.09 -> 0.21 us, 16x16 1.12 -> 0.19 us; 120 uneven lattices of
+// 4-16 a side 27.3 -> 4.8 ms; the operator, 64 samples of 9x9, 1000 rounds, with
+// set-up 2.05 -> 0.31 ms.  On the way: branches around site fallback and claims
+// 0.40 us a round, a branch in the barrier, around the lattice stores and a load
+// of the claim each round 0.26 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -84,15 +85,17 @@ __device__ __forceinline__ int accept_limit(uint32_t x, const uint32_t* acc_thr)
 
 struct PreSync {
   int threads;
-  __device__ __forceinline__ void operator()() const
-  {
-    if (threads == 32) {
-      __syncwarp();
-    } else {
-      asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
-    }
-  }
+  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 };
+
+// A store under a predicate; without it the compiler branches around a pair.
+__device__ __forceinline__ void store_if(bool p, uint32_t* a, uint32_t v)
+{
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}" ::"r"(
+                 static_cast<uint32_t>(p)),
+               "r"(static_cast<uint32_t>(__cvta_generic_to_shared(a))), "r"(v)
+               : "memory");
+}
 
 // A sample's walk: where its pieces lie and its parameters.
 struct PreWalk {
@@ -178,7 +181,7 @@ struct Copy {
 // stops the walker (wl.cu:522-529) and leaves its energy in E.  Every thread of
 // the CTA's first p.threads calls it.  On return both copies of the histogram
 // hold all visits.
-template <bool kTwo, bool kRange>
+template <bool kTwo, bool kRange, bool kKeys>
 __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, int w, bool live, uint64_t key,
                                          uint64_t subseq, uint64_t& pos, int& E, uint32_t& s0)
 {
@@ -198,6 +201,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   if (kRange) ok = ok && E >= p.e_min && E <= p.e_max;
   int io = ok ? E - p.e_min : spare;
   int hit_before = spare;
+  int e_start = io;     // batched walk: the one bin visited without a move into it
   int want = -1;        // coarse bin claimed in the round before
   bool claims = false;  // a lane of this warp has one
   uint32_t claim_key = 1u << 10;  // of this round
@@ -239,7 +243,10 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   // this round's move when it is still empty (`key`: this round's).  What is
   // rare (a site next to a cell edge, a draw next to a threshold, an empty
   // bin) is settled in one warp-uniform block: the rest has no branch.
-  auto prepare = [&](uint32_t x_site, uint32_t x_acc, bool moved, uint32_t key_now) {
+  // fresh: the bin moved into had no visit before this round.  In a batched walk
+  // only such bins, and the one all walkers start in, can lie in an empty
+  // coarse bin; the operator's histogram may hold earlier visits.
+  auto prepare = [&](uint32_t x_site, uint32_t x_acc, bool moved, bool fresh, uint32_t key_now) {
     const uint64_t xi = static_cast<uint64_t>(x_site) * static_cast<uint32_t>(X);
     const uint64_t xj = static_cast<uint64_t>(static_cast<uint32_t>(xi)) * static_cast<uint32_t>(Y);
     const bool edge = static_cast<uint32_t>(xj) + site_thr < 2u * site_thr;
@@ -249,19 +256,27 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
     const float big = v + 0x1.8p23f, away = v - (big - 0x1.8p23f);
     limit = __float_as_int(big) - 0x4B400000 - (away < 0.0f ? 1 : 0);
     const bool close = fabsf(away) < 2.0f * kLogAbsErr;
-    const int q = min(len_one ? io : static_cast<int>(__umulhi(static_cast<uint32_t>(io), len_magic)), p.n_int - 1);
-    const bool empty = moved && p.claim[q] >= key_now;  // or claimed in this round
+    auto coarse = [&]() {
+      return min(len_one ? io : static_cast<int>(__umulhi(static_cast<uint32_t>(io), len_magic)), p.n_int - 1);
+    };
+    bool empty = kRange ? moved & (p.claim[coarse()] >= key_now) : moved & (fresh | (io == e_start));
     claims = false;
     want = -1;
-    if (__any_sync(0xFFFFFFFFu, edge || close || empty)) {
+    if (__any_sync(0xFFFFFFFFu, edge | close | empty)) {
       if (edge) {
         const uint32_t site = static_cast<uint32_t>(site_exact(x_site, site_scale)), i = site / static_cast<uint32_t>(Y);
         propose(i, site - i * static_cast<uint32_t>(Y));
       }
       if (close) limit = accept_limit(x_acc, p.acc_thr);
       if (empty) {
-        atomicMin(&p.claim[q], key_now | static_cast<uint32_t>(w));
-        want = q;
+        const int q = coarse();
+        empty = p.claim[q] >= key_now;  // empty, or claimed in this round
+        if (empty) {
+          atomicMin(&p.claim[q], key_now | static_cast<uint32_t>(w));
+          want = q;
+        } else if (io == e_start) {
+          e_start = -1;
+        }
       }
       claims = __any_sync(0xFFFFFFFFu, empty);
     }
@@ -300,12 +315,10 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
     }
     const uint32_t h_old = now[io], h_new = now[can ? in : spare];
     beside();
-    const bool acc = can && static_cast<int>(h_new - h_old) <= limit;
-    if (acc) {
-      lat[wa] = na;
-      lat[wb] = nb;
-      if constexpr (kTwo) lat[wc] = nc;
-    }
+    const bool acc = can & (static_cast<int>(h_new - h_old) <= limit);
+    store_if(acc, lat + wa, na);
+    store_if(acc, lat + wb, nb);
+    if constexpr (kTwo) store_if(acc, lat + wc, nc);
     io = acc ? in : io;
     s0 ^= acc ? first_site : 0u;
     const int hit = ok ? io : spare;
@@ -315,13 +328,23 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
     if (kRange && ok) pos += 2;
     const uint32_t key_now = claim_key;
     claim_key += 1u << 10;
-    prepare(x_site, x_acc, acc, key_now);
+    prepare(x_site, x_acc, acc, h_new == 0u, key_now);
   };
 
   // four draws at a time from an even position (a fresh walk's is 0)
   uint64_t blk = pos >> 2;
+  // kKeys: round keys in registers, 18 additions fewer per block
+  uint32_t ka[10], kb[10];
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    ka[r] = k0 + static_cast<uint32_t>(r) * kPhiloxWeylA;
+    kb[r] = k1 + static_cast<uint32_t>(r) * kPhiloxWeylB;
+    if constexpr (kKeys) asm volatile("" : "+r"(ka[r]), "+r"(kb[r]));
+  }
   auto block = [&]() {
-    const uint4 c = philox10(static_cast<uint32_t>(blk), static_cast<uint32_t>(blk >> 32), s_lo, s_hi, k0, k1);
+    uint4 c = make_uint4(static_cast<uint32_t>(blk), static_cast<uint32_t>(blk >> 32), s_lo, s_hi);
+#pragma unroll
+    for (int r = 0; r < 10; ++r) c = philox_round(c, ka[r], kb[r]);
     ++blk;
     return c;
   };
@@ -336,8 +359,9 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
     return o;
   };
   uint4 a = four();
-  prepare(a.x, a.y, false, claim_key);
+  prepare(a.x, a.y, false, false, claim_key);
   int left = p.n_iter;
+#pragma unroll 2
   for (; left >= 2; left -= 2) {
     uint4 b;
     round(Copy<0>{}, a.z, a.w, [&] { b = four(); });

@@ -26,6 +26,15 @@ constexpr uint32_t kPhiloxMulB = 0xCD9E8D57u;
 constexpr uint32_t kPhiloxWeylA = 0x9E3779B9u;
 constexpr uint32_t kPhiloxWeylB = 0xBB67AE85u;
 
+// One Philox4x32 round under the key (k0, k1).
+__device__ __forceinline__ uint4 philox_round(uint4 c, uint32_t k0, uint32_t k1)
+{
+  const uint64_t pa = static_cast<uint64_t>(kPhiloxMulA) * c.x;
+  const uint64_t pb = static_cast<uint64_t>(kPhiloxMulB) * c.z;
+  return make_uint4(static_cast<uint32_t>(pb >> 32) ^ c.y ^ k0, static_cast<uint32_t>(pb),
+                    static_cast<uint32_t>(pa >> 32) ^ c.w ^ k1, static_cast<uint32_t>(pa));
+}
+
 // kRounds Philox4x32 rounds applied to the state c, the first of them under
 // the key (k0, k1); the key advances by the Weyl constants every round.
 template <int kRounds>
@@ -33,14 +42,7 @@ __device__ __forceinline__ uint4 philox_rounds(uint4 c, uint32_t k0, uint32_t k1
 {
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
-    const uint64_t pa = static_cast<uint64_t>(kPhiloxMulA) * c.x;
-    const uint64_t pb = static_cast<uint64_t>(kPhiloxMulB) * c.z;
-    const uint32_t n0 = static_cast<uint32_t>(pb >> 32) ^ c.y ^ k0;
-    const uint32_t n2 = static_cast<uint32_t>(pa >> 32) ^ c.w ^ k1;
-    c.y = static_cast<uint32_t>(pb);
-    c.w = static_cast<uint32_t>(pa);
-    c.x = n0;
-    c.z = n2;
+    c = philox_round(c, k0, k1);
     k0 += kPhiloxWeylA;
     k1 += kPhiloxWeylB;
   }
