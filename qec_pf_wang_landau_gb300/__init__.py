@@ -240,17 +240,18 @@ class Context:
         self._check("wlg_solve_raw", lib().wlg_solve_raw(self._h, C.cast(arr, P), n, C.cast(res, P),
                                                           ws.ctypes.data_as(P), we.ctypes.data_as(P),
                                                           raw.ctypes.data_as(P), cap, off.ctypes.data_as(P)))
+        # the windows of a problem share one copy of its values
         out, wpos = [], 0
+        start = off.tolist()
         for p, q in enumerate(problems):
             s = ws[wpos:wpos + q.intervals].copy()
             e = we[wpos:wpos + q.intervals].copy()
             wpos += q.intervals
-            wins, pos = [], int(off[p])
+            wins = []
             if res[p].status in (WLG_OK, WLG_ERR_TIMEOUT):
-                for b in range(q.intervals):
-                    ln = int(e[b] - s[b] + 1)
-                    wins.append(raw[pos:pos + ln].copy())
-                    pos += ln
+                ends = np.cumsum(e - s + 1).tolist()
+                v = raw[start[p]:start[p] + ends[-1]].copy()
+                wins = [v[a:b] for a, b in zip([0] + ends, ends)]
             out.append((res[p], s, e, wins))
         return out
 

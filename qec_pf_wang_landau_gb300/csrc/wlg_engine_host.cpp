@@ -998,16 +998,6 @@ struct HostExec final : Exec {
   wlg_status buffer(Slot, size_t, void**) override { return WLG_ERR_INVALID; }
 };
 
-// Dense walker-0 log g of window b (zeros where the lattice cannot reach).
-void dense_window(const MainDesc& d, const std::vector<double>& out, const std::vector<int>& win, int b,
-                  std::vector<double>& dense)
-{
-  const int s = win[d.off_win + b], e = win[d.off_win + d.I + b];
-  const int base = win[d.off_win + 2 * d.I + b], len = win[d.off_win + 3 * d.I + b];
-  dense.assign(static_cast<size_t>(e - s + 1), 0.0);
-  for (int c = 0; c < len; ++c) dense[base + (c << d.lg) - s] = out[d.off_out + static_cast<long long>(b) * d.L + c];
-}
-
 }  // namespace
 
 extern "C" {
@@ -1140,28 +1130,42 @@ wlg_status raw_windows(Exec& ex, const wlg_problem* problems, int n, const Prepa
                        const std::vector<double>& out, const std::vector<int>& win, int* win_start, int* win_end,
                        double* raw_log_g, long long raw_capacity, long long* raw_offset)
 {
-  long long pos = 0;
   std::vector<int> slot(static_cast<size_t>(n), -1);
   for (size_t i = 0; i < prep.main.size(); ++i) slot[prep.main_problem[i]] = static_cast<int>(i);
+  std::vector<long long> at(static_cast<size_t>(n) + 1, 0);  // first value of each problem
   long long wpos = 0;
   for (int p = 0; p < n; ++p) {
-    if (raw_offset != nullptr) raw_offset[p] = pos;
+    if (raw_offset != nullptr) raw_offset[p] = at[p];
     const int I = problems[p].intervals;
+    const bool have = !prep.starts[p].empty();
+    at[p + 1] = at[p];
     for (int b = 0; b < I; ++b) {
-      const bool have = !prep.starts[p].empty();
       if (win_start != nullptr) win_start[wpos + b] = have ? prep.starts[p][b] : 0;
       if (win_end != nullptr) win_end[wpos + b] = have ? prep.ends[p][b] : -1;
+      if (slot[p] >= 0) at[p + 1] += prep.ends[p][b] - prep.starts[p][b] + 1;
     }
     wpos += I;
-    if (slot[p] < 0) continue;
+    if (at[p + 1] > raw_capacity) return fail(ex, WLG_ERR_CAPACITY, "raw output");
+  }
+  if (raw_log_g == nullptr) return WLG_OK;
+  // zeros where the lattice cannot reach; problems are independent
+  const auto one = [&](int p) {
+    if (slot[p] < 0) return;
     const MainDesc& d = prep.main[slot[p]];
-    std::vector<double> dense;
+    double* dst = raw_log_g + at[p];
+    std::fill(dst, raw_log_g + at[p + 1], 0.0);
     for (int b = 0; b < d.I; ++b) {
-      dense_window(d, out, win, b, dense);
-      if (pos + static_cast<long long>(dense.size()) > raw_capacity) return fail(ex, WLG_ERR_CAPACITY, "raw output");
-      if (raw_log_g != nullptr) std::memcpy(raw_log_g + pos, dense.data(), dense.size() * sizeof(double));
-      pos += static_cast<long long>(dense.size());
+      const int s = win[d.off_win + b], e = win[d.off_win + d.I + b];
+      const int base = win[d.off_win + 2 * d.I + b], len = win[d.off_win + 3 * d.I + b];
+      const double* src = out.data() + d.off_out + static_cast<long long>(b) * d.L;
+      for (int c = 0; c < len; ++c) dst[base + (c << d.lg) - s] = src[c];
+      dst += e - s + 1;
     }
+  };
+  if (ex.pool != nullptr) {
+    ex.pool->run(n, 8, one);
+  } else {
+    for (int p = 0; p < n; ++p) one(p);
   }
   return WLG_OK;
 }
