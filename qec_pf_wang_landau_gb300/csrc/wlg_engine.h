@@ -247,8 +247,8 @@ WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, boo
   o = align16(o + 4 * I);
   t.off_flat = o;
   o = align16(o + 4 * I);
-  t.off_stab = o;  // per window: averaging is a fixed point [I], then changed-in-this-pass [I]
-  o = align16(o + 8 * I);
+  t.off_stab = o;  // per window: averaging is a fixed point [I], changed in this pass [I], limits exceeded [I]
+  o = align16(o + (tight ? 8 : 12) * I);
   t.off_win = o;
   o = align16(o + 4 * 5 * I);
   t.off_misc = o;

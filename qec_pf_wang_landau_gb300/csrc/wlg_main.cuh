@@ -60,6 +60,11 @@ namespace {
 
 constexpr double kE = 2.718281828459045;  // std::numbers::e, mainrun.cu:56
 
+template <int kC>
+struct Count {
+  static constexpr int value = kC;
+};
+
 struct Team {
   int size;  // threads
   int id;    // barrier id (1..15) or 0 for a single warp
@@ -139,6 +144,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   // suspended run: a resumed one recomputes one pass, with the same result.
   int* stab = reinterpret_cast<int*>(base + lay.off_stab);
   int* chg = stab + d.I;
+  [[maybe_unused]] int* above = stab + 2 * d.I;
   int* win = reinterpret_cast<int*>(base + lay.off_win);  // start, end, base, Lb, E0
   int* misc = reinterpret_cast<int*>(base + lay.off_misc);
   unsigned long long* new_key = reinterpret_cast<unsigned long long*>(misc + 4);
@@ -249,7 +255,13 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   Stream& rng = wk.rng;
   rng.init(d.key_wl, static_cast<uint64_t>(t), 0);
   const bool keys_differ = d.key_ex != static_cast<uint64_t>(d.key_wl);
-  const double reset_lim = exp(d.beta);  // wl.cu:609
+  // what a factor exceeds: 2 the limit that resets a window (wl.cu:609), 1 the
+  // loop's (mainrun.cu:243); kept per window, as factors rarely change (the
+  // tight layout has no room for it)
+  const double reset_lim = exp(d.beta);
+  auto limits = [&](double f) { return (f > reset_lim ? 2 : 0) + (f - d.loop_lim > 1e-10 ? 1 : 0); };
+  if constexpr (!kTight)
+    for (int q = t; q < I; q += P) above[q] = limits(kE);
   long long outer = 0;
   long long counter = 1;
   int status = WLG_OK;
@@ -260,6 +272,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
     if (t < I) {
       fwin[t] = reinterpret_cast<const double*>(st + sl.off_f)[t];
       lnfw[t] = log(fwin[t]);
+      if constexpr (!kTight) above[t] = limits(fwin[t]);
       cond[t] = reinterpret_cast<const int*>(st + sl.off_cond)[t];
     }
     perm[t] = reinterpret_cast<const int*>(st + sl.off_perm)[t];
@@ -292,6 +305,15 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   const uint32_t tab_a = shared_addr(base + lay.off_tab);
   const SweepTeam common{d, P, tab_a, tab_a + (kTable ? 16 * d.N : align16(8 * d.Y)), Jr_s, Jd_s, JR, JD};
   const bool w_pow2 = (W & (W - 1)) == 0;
+  // the exchange takes at most W draws of a walker, from its ring where that
+  // holds them and the keys agree
+  const bool ring_draws = !kTight && !keys_differ && W <= kRingAhead;
+  auto draw = [&]() {
+    if constexpr (!kTight) {
+      if (ring_draws) return lds_u32(wk.ring_a + (static_cast<uint32_t>(rng.pos++) * 128u & 2047u));
+    }
+    return rng.raw();
+  };
   if (resumed && t == 0) misc[7] = static_cast<int>(outer + 1);  // finished windows get one averaging pass
   int launch_outer = 0;  // outer iterations of this launch
   bool suspended = false;
@@ -302,6 +324,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       status = WLG_ERR_TIMEOUT;
       break;
     }
+    const bool exchange_next = counter % d.exch_every == 0;
     // ---- WL sweep (wl.cu:1077-1175)
     const unsigned wmask = __ballot_sync(0xFFFFFFFFu, live);
     if (live) {
@@ -326,31 +349,53 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
         unsigned long long sum = 0;
         int cnt = 0;
         const int cb = (bb - d.e_min) >> d.lg;
-#pragma unroll 2
-        for (int c = 0; c < len; ++c) {
-          const float2 v = pair[c * P + t];
-          const uint32_t k = static_cast<uint32_t>(v.y);
-          const uint32_t h = H[c * P + t] + k;
-          double g = G[c * P + t];
-          const bool on = kTight ? mask_has(mask, cb + c) : v.x == v.x;
-          if (k != 0) {
-            g = add_times<false>(g, lnf, k);
-            G[c * P + t] = g;
-            H[c * P + t] = h;
+        // four bins at a time, so that their loads and integer chains overlap
+        // (200 -> 70 cycles a bin); what add_times_in_binade leaves goes one by one
+        const Addend add = split_addend(lnf);
+        auto fold_bins = [&](int c, auto count) {
+          constexpr int kN = decltype(count)::value;
+          float2 v[kN];
+          double g[kN];
+          uint32_t h[kN], k[kN];
+          unsigned slow = 0;
+#pragma unroll
+          for (int u = 0; u < kN; ++u) {
+            v[u] = pair[(c + u) * P + t];
+            g[u] = G[(c + u) * P + t];
+            h[u] = H[(c + u) * P + t];
           }
-          const float a = shadow_split(g, wk.gs);
-          pair[c * P + t] = make_float2(kTight || on ? a : v.x, 0.0f);
-          if (on) {
-            mn = min(mn, h);
-            sum += h;
-            ++cnt;
-            wk.amax = fmaxf(wk.amax, fabsf(a));
-            wk.ghi = max(wk.ghi, __double2hiint(g));
-          } else if (kTight) {
-            wk.amax = fmaxf(wk.amax, fabsf(a));
-            wk.ghi = max(wk.ghi, __double2hiint(g));
+#pragma unroll
+          for (int u = 0; u < kN; ++u) {
+            k[u] = static_cast<uint32_t>(v[u].y);
+            h[u] += k[u];
+            bool ok = true;
+            const double sum = add_times_in_binade(g[u], add, k[u], ok);
+            slow |= k[u] != 0 && !ok ? 1u << u : 0u;
+            g[u] = k[u] != 0 && ok ? sum : g[u];
           }
-        }
+          if (slow != 0) {
+#pragma unroll
+            for (int u = 0; u < kN; ++u)
+              if ((slow >> u) & 1u) g[u] = add_times<false>(g[u], lnf, k[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < kN; ++u) {
+            const int q = (c + u) * P + t;
+            const bool on = kTight ? mask_has(mask, cb + c + u) : v[u].x == v[u].x;
+            const float a = shadow_split(g[u], wk.gs);
+            pair[q] = make_float2(kTight || on ? a : v[u].x, 0.0f);
+            G[q] = g[u];
+            H[q] = h[u];
+            mn = on ? min(mn, h[u]) : mn;
+            sum += on ? h[u] : 0u;
+            cnt += on ? 1 : 0;
+            wk.amax = kTight || on ? fmaxf(wk.amax, fabsf(a)) : wk.amax;
+            wk.ghi = kTight || on ? max(wk.ghi, __double2hiint(g[u]) & 0x7FFFFFFF) : wk.ghi;
+          }
+        };
+        int c = 0;
+        for (; c + 4 <= len; c += 4) fold_bins(c, Count<4>{});
+        for (; c < len; ++c) fold_bins(c, Count<1>{});
         if (last && cnt > 0) {
           // min >= alpha * (sum / cnt): in FP32 unless the sides are close
           const float have = static_cast<float>(mn) * static_cast<float>(cnt);
@@ -361,7 +406,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
           if (is_flat && atomicAdd(&flat[b], 1) == W - 1) misc[3] = static_cast<int>(outer + 1);
         }
       };
-      wl_sweep<kStore, kTight, false>(common, wk, wmask, d.n_iter, frozen, lnf, log_g, is_bad, new_energy, fold);
+      wl_sweep<kStore, kTight, false>(common, wk, wmask, d.n_iter, frozen, lnf, exchange_next && ring_draws ? W : 0, log_g, is_bad, new_energy, fold);
     }
     team.sync();
     ++outer;
@@ -408,22 +453,23 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       if (cond[t] == 0 && flat[t] == W) {
         fwin[t] = sqrt(fwin[t]);
         lnfw[t] = log(fwin[t]);
+        if constexpr (!kTight) above[t] = limits(fwin[t]);
         cond[t] = 1;
       }
-      const double f = fwin[t];
-      if (cond[t] == 1 && f > reset_lim) cond[t] = 0;
+      const int over = kTight ? limits(fwin[t]) : above[t];
+      if (cond[t] == 1 && over >= 2) cond[t] = 0;
       stab[t] = cond[t] == 1 && (stab[t] != 0 || chg[t] == 0) ? 1 : 0;
       chg[t] = 0;
       flat[t] = 0;
       if (cond[t] == 1 && stab[t] == 0) misc[7] = stamp + 1;
       if (cond[t] != 1) misc[6] = stamp;
-      if (f - d.loop_lim > 1e-10) misc[2] = stamp;
+      if ((over & 1) != 0) misc[2] = stamp;
     }
     team.sync();
     const bool done = misc[6] != stamp;
     const bool stop = misc[2] != stamp;  // the largest factor is at the limit
     // ---- replica exchange (wl.cu:785-890)
-    if (!done && counter % d.exch_every == 0) {
+    if (!done && exchange_next) {
       if (live) {
         E_s[t] = E;
         if constexpr (kReg) {
@@ -432,7 +478,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
         }
         if (keys_differ) {
           rng.init(d.key_ex, static_cast<uint64_t>(t), rng.pos);
-        } else {
+        } else if (!ring_draws) {
           rng.refill();
         }
       }
@@ -445,7 +491,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
         if (active && w == 0) {  // Fisher-Yates by the window's first walker
           for (int i = W - 1; i > 0; --i) {
             // trunc(u (i + 0.999999)), as the sweep's site among i + 1
-            const uint32_t x = rng.raw(), n1 = static_cast<uint32_t>(i) + 1u, thr = n1 * 2048u + 16384u;
+            const uint32_t x = draw(), n1 = static_cast<uint32_t>(i) + 1u, thr = n1 * 2048u + 16384u;
             int r = static_cast<int>(__umulhi(x, n1));
             if (x * n1 + thr < 2u * thr) r = main_site_exact(x, i + 0.999999);
             const int tmp = perm[t + i];
@@ -463,13 +509,24 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
             const double gi_y = G[((eo - bb) >> d.lg) * P + t];
             const double gj_y = G[((eo - nb) >> d.lg) * P + o];
             const double gj_x = G[((et - nb) >> d.lg) * P + o];
-            if (exchange_accepts(rng.raw(), gi_x - gi_y, gj_y - gj_x)) {
+            if (exchange_accepts(draw(), gi_x - gi_y, gj_y - gj_x)) {
               E_s[t] = eo;
               E_s[o] = et;
-              for (int q = 0; q < nw; ++q) {
-                const uint32_t a = lat_s[q * P + t];
-                lat_s[q * P + t] = lat_s[q * P + o];
-                lat_s[q * P + o] = a;
+              // four words at a time: their loads overlap
+              for (int q = 0; q < nw; q += 4) {
+                uint32_t a[4], c[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const int r = min(q + u, nw - 1) * P;
+                  a[u] = lat_s[r + t];
+                  c[u] = lat_s[r + o];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const int r = min(q + u, nw - 1) * P;
+                  lat_s[r + t] = c[u];
+                  lat_s[r + o] = a[u];
+                }
               }
             }
           }

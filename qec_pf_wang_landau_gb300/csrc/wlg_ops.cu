@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
       G[c << lg] = add_times<true>(G[c << lg], lnf, n);
     }
   };
-  wl_sweep<kStore, false, true>(team, wk, wmask, a.n_iter, frozen, lnf, log_g, is_bad, new_energy, fold);
+  wl_sweep<kStore, false, true>(team, wk, wmask, a.n_iter, frozen, lnf, 0, log_g, is_bad, new_energy, fold);
   // lattices: rows as they are; bonds down column 0, then along each row
   uint32_t edge = wk.s0;
   for (int i = 0; i < X; ++i) {

@@ -97,12 +97,23 @@ __device__ __noinline__ bool accept_exact(uint32_t x2, double g, double g_new)
 // exactly half-way between two of them.  Additions that leave the binade, ties
 // and |g| < c take the FP64 addition; they are few (a tie needs the last
 // log2(|g| / c) bits of c to be 10..0).
+// Where no addition rounds at all (ln f = 1 on whole numbers, until the first
+// average: bins cross binades all the time then) one fused multiply-add is the sum.
 template <bool kSigned>
 __device__ __forceinline__ double add_times(double g, double c, uint32_t n)
 {
   const unsigned long long bc = __double_as_longlong(c);
   const unsigned long long m = (bc & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
   const int ec = static_cast<int>(bc >> 52);
+  {
+    // exact: c and g are multiples of the largest partial sum's unit
+    const double sum = fma(static_cast<double>(n), c, g);
+    const int eg = (__double2hiint(g) >> 20) & 0x7FF, es = (__double2hiint(sum) >> 20) & 0x7FF, top = max(eg, es);
+    const unsigned long long below = (1ull << (min(top - eg, 52))) - 1;
+    if (top - ec <= __ffsll(static_cast<long long>(m)) - 1 && (__double_as_longlong(g) & below) == 0 &&
+        (eg > 0 || g == 0.0) && top - (eg > 0 ? eg : top) <= 52)
+      return sum;
+  }
   while (n > 0) {
     unsigned long long bg = __double_as_longlong(g);
     const bool neg = kSigned && (bg >> 63) != 0;
@@ -131,6 +142,34 @@ __device__ __forceinline__ double add_times(double g, double c, uint32_t n)
     --n;
   }
   return g;
+}
+
+// add_times without a loop, for n < 2^31 and g >= 0: the sum when it keeps g's
+// exponent and no tie or g < c comes up, else ok = false.  m, ec: significand and
+// exponent field of c (split_addend); integer operations only, about 25.
+struct Addend {
+  unsigned long long m;
+  int ec;
+};
+__device__ __forceinline__ Addend split_addend(double c)
+{
+  const unsigned long long b = __double_as_longlong(c);
+  return Addend{(b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull, static_cast<int>(b >> 52)};
+}
+__device__ __forceinline__ double add_times_in_binade(double g, const Addend& c, uint32_t n, bool& ok)
+{
+  const unsigned long long bg = __double_as_longlong(g);
+  const int sh = static_cast<int>(bg >> 52) - c.ec;
+  const unsigned long long cut = c.m << ((64 - sh) & 63);  // the bits of c below g's grid, from the top
+  const unsigned long long step = (c.m >> (sh & 63)) + (cut > 0x8000000000000000ull ? 1u : 0u);
+  // n steps: step < 2^52 and n < 2^31 as two 32-bit products; up must stay
+  // below what is left of the binade, so its high word below 2^20
+  const unsigned long long low = static_cast<unsigned long long>(static_cast<uint32_t>(step)) * n;
+  const unsigned long long high = (step >> 32) * n + (low >> 32);
+  const unsigned long long up = high << 32 | static_cast<uint32_t>(low);
+  ok = (sh >= 1) & (sh <= 52) & (c.ec > 0) & (cut != 0x8000000000000000ull) & (high < (1u << 20)) &
+       (up <= 0xFFFFFFFFFFFFFull - (bg & 0xFFFFFFFFFFFFFull));
+  return __longlong_as_double(static_cast<long long>(bg + up));
 }
 
 // Split and shadow of a log g of either sign (kSigned), else of g >= 0.
@@ -290,6 +329,8 @@ __device__ __forceinline__ uint32_t bond_word(uint32_t r, uint32_t below, uint32
   return h | v << 16;
 }
 
+constexpr int kRingAhead = kRingSlots - 4 + 1;  // a block is added while it fits
+
 // What the team's walkers have in common.
 struct SweepTeam {
   const MainDesc& d;  // lattice, draws and energy step
@@ -332,6 +373,7 @@ struct Walker {
 };
 
 // n_iter steps of the lane's walker; the lanes of wmask call it together.
+// ahead: draws to be left in the ring (at most kRingAhead).
 // kSign (the caller's arrays): keep the spin of site 0, which bond words alone
 // do not tell, and take log g of either sign.
 // log_g(c): FP64 log g of bin c; is_bad(E): the pre-run never saw E
@@ -340,7 +382,7 @@ struct Walker {
 // walker's bins to histogram and log g and clears them.
 template <int kStore, bool kTight, bool kSign, class LogG, class IsBad, class NewEnergy, class Fold>
 __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& wk, unsigned wmask, int n_iter, bool frozen,
-                                         double lnf, LogG log_g, IsBad is_bad, NewEnergy new_energy, Fold fold)
+                                         double lnf, int ahead, LogG log_g, IsBad is_bad, NewEnergy new_energy, Fold fold)
 {
   constexpr bool kTable = kStore == kStoreTable;
   constexpr bool kReg = kStore == kStoreReg || kTable;
@@ -482,7 +524,7 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
       philox_store();
     };
     asm volatile("" ::: "memory");
-    while (__any_sync(wmask, static_cast<int>(fill - pos) <= 12 * 128)) produce();
+    while (__any_sync(wmask, static_cast<int>(fill - pos) < 8 * 128)) produce();
     uint32_t xa, xb, xc, xd;  // the draws at pos .. pos + 3
     auto reload = [&]() {
       xa = ring_get(pos);
@@ -708,7 +750,7 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
     for (;;) {
       if (rem <= 0) thr = kInf;
       if (!__any_sync(wmask, rem > 0 && !stopped)) break;
-      produce();
+      if (__any_sync(wmask, static_cast<int>(fill - pos) < 8 * 128)) produce();
       step(none, none);
       if (__any_sync(wmask, thr == kInf && rem > 0 && !stopped)) exact_step();
     }
@@ -716,6 +758,8 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
     const int c_last = kTight ? static_cast<int>(cur) : static_cast<int>((cur - bin0) / bin_bytes);
     E = bb + c_last * (1 << d.lg) + e_off;
     rng.pos = pos0 + ((pos - pos_start) >> 7);
+    if (left == 0)
+      while (__any_sync(wmask, static_cast<int>(fill - pos) < ahead * 128)) produce();
     fold(n_c, c_last, left == 0);
   }
 }
