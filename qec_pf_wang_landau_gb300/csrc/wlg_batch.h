@@ -178,7 +178,11 @@ constexpr int kVariantGlobal = 8;  // log g and histogram in global memory
 constexpr int kVariantTight = 16;  // see team_layout; always with kVariantGlobal
 constexpr int kSmemBytes = 227 * 1024;
 
+// in bits 8 and up: CTAs of the cluster a problem is spread over, 0 or 1 none
+constexpr int kVariantRanks = 256;
+
 inline int variant_store(int variant) { return variant & 7; }
+inline int variant_ranks(int variant) { return variant >= kVariantRanks ? variant / kVariantRanks : 1; }
 
 // The form wlg.h reports: 0 lattice and log g in shared memory, 1 lattice in a
 // register, 2 the register with a neighbour table, 3 log g in global memory.

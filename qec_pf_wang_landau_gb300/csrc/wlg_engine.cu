@@ -267,6 +267,7 @@ wlg_status launch_pre_batch(const PreDesc* d_descs, int n, int threads, int smem
 
 MainFn main_fn(int variant, int cta_threads)
 {
+  if (variant_ranks(variant) > 1) return main_fn_cluster(variant_store(variant));
   const bool tight = (variant & kVariantTight) != 0;
   if (cta_threads <= 256) return main_fn_256(variant_store(variant), tight);
   if (cta_threads <= 512) return main_fn_512(variant_store(variant), tight);
@@ -280,6 +281,22 @@ int main_batch_capacity(int variant, int cta_threads, int smem)
   MainFn fn = main_fn(variant, cta_threads);
   int per_sm = 0;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
+  const int ranks = variant_ranks(variant);
+  if (ranks > 1) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ranks);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(ranks));
+    cfg.blockDim = dim3(static_cast<unsigned>(cta_threads));
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) return 0;
+    return clusters * ranks;
+  }
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, cta_threads, smem) != cudaSuccess) return 0;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -298,10 +315,23 @@ wlg_status launch_main_batch(int variant, const MainDesc* d_descs, const int* d_
   const int smem = team_bytes * teams_per_cta;
   MainFn fn = main_fn(variant, threads);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return WLG_ERR_CUDA;
-  fn<<<grid, threads, smem, s>>>(d_descs, d_order, n, team_size, team_bytes, (variant & kVariantGlobal) != 0 ? 1 : 0,
-                                 d_next, gpool, gslot_doubles, Jpool, latpool, winpool, maskpool, outpool, results,
-                                 statepool);
-  return launch_status();
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = s;
+  if (variant_ranks(variant) > 1) {
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(variant_ranks(variant));
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+  const cudaError_t e =
+    cudaLaunchKernelEx(&cfg, fn, d_descs, d_order, n, team_size, team_bytes, (variant & kVariantGlobal) != 0 ? 1 : 0,
+                       d_next, gpool, gslot_doubles, Jpool, latpool, winpool, maskpool, outpool, results, statepool);
+  return e == cudaSuccess ? launch_status() : WLG_ERR_CUDA;
 }
 
 }  // namespace wlg

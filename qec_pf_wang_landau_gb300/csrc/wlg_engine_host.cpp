@@ -719,6 +719,32 @@ namespace {
 // then the histogram (32 bits) [L][team].
 long long pool_slice(int L, int team) { return (3LL * L * team + 1) / 2; }
 
+// CTAs a problem is spread over when each may take `spread`: no team smaller than
+// four warps, one per partition of an SM, and a window at least in each.
+int problem_ranks(const MainDesc& d, int spread)
+{
+  int r = 1;
+  while (r < spread && d.team / (2 * r) >= 128 && d.I >= 2 * r) r *= 2;
+  return r;
+}
+
+// Threads of one of the teams a problem is spread over.
+int rank_team(const MainDesc& d, int ranks) { return round32((d.I + ranks - 1) / ranks * d.W); }
+
+// The largest spread (up to 8) that leaves every team an SM of its own.  A
+// problem of 512 walkers on one SM has four warps on each partition, which share
+// its issue slots; on four SMs each warp has its own.
+int spread_ranks(const Prepared& prep, int sms)
+{
+  int spread = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    int teams = 0;
+    for (const MainDesc& d : prep.main) teams += problem_ranks(d, s);
+    if (teams <= sms) spread = s;
+  }
+  return spread;
+}
+
 constexpr int kTimedEpoch = 4;  // outer iterations per launch under a time limit
 
 // The main run of a prepared batch: one persistent launch per (form, team
@@ -752,7 +778,17 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex.device);
   // one launch per (form, team size); the form by lattice storage (fit_form)
   std::map<std::pair<int, int>, std::vector<int>> groups;
-  for (int i = 0; i < m; ++i) groups[{wlg::kernel_variant(prep.main[i], prep.main[i].team), prep.main[i].team}].push_back(i);
+  const int spread = time_limit_s > 0 ? 1 : spread_ranks(prep, sms);
+  for (int i = 0; i < m; ++i) {
+    const MainDesc& d = prep.main[i];
+    const int ranks = problem_ranks(d, spread), team = rank_team(d, ranks);
+    const int variant = wlg::kernel_variant(d, team);
+    if (ranks > 1 && (variant & wlg::kVariantTight) == 0) {
+      groups[{variant | ranks * wlg::kVariantRanks, team}].push_back(i);
+    } else {
+      groups[{wlg::kernel_variant(d, d.team), d.team}].push_back(i);
+    }
+  }
   // Longest problems first (larger lattices take more outer iterations of
   // longer steps): the groups' launches are issued, and each group's queue
   // is ordered, by decreasing lattice size, so the batch's longest serial
@@ -777,7 +813,7 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
       Lmax = std::max(Lmax, prep.main[i].L);
     }
     for (int i : idx)
-      if (wlg::admission_bytes(prep.main[i], team) > wlg::kSmemBytes)
+      if (wlg::admission_bytes(prep.main[i], prep.main[i].team) > wlg::kSmemBytes)
         return fail(ex, WLG_ERR_INVALID, "problem state exceeds shared memory");
     int per_cta = team <= 256 ? 256 / team : 1;
     per_cta = std::min(per_cta, (227 * 1024) / bytes);
@@ -786,7 +822,8 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     // than packing them into few CTAs
     per_cta = std::min(per_cta, static_cast<int>(idx.size()) / (2 * sms));
     per_cta = std::max(per_cta, 1);
-    if (ex.per_cta != nullptr) {
+    if (wlg::variant_ranks(variant) > 1) per_cta = 1;
+    else if (ex.per_cta != nullptr) {
       auto it = ex.per_cta->find({variant, team});
       if (it != ex.per_cta->end()) {
         per_cta = std::max(1, std::min(it->second, team <= 256 ? 256 / team : 1));
@@ -828,7 +865,8 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   std::vector<long long> pool_later(launches.size() + 1, 0);  // one CTA's slices of each later launch
   for (size_t g = launches.size(); g-- > 1;) {
     const bool global = (std::get<0>(launches[g]) & wlg::kVariantGlobal) != 0;
-    const long long cta = std::get<3>(launches[g]) * pool_slice(std::get<6>(launches[g]), std::get<1>(launches[g]));
+    const long long cta = wlg::variant_ranks(std::get<0>(launches[g])) * std::get<3>(launches[g]) *
+                          pool_slice(std::get<6>(launches[g]), std::get<1>(launches[g]));
     pool_later[g - 1] = pool_later[g] + (global ? cta : 0);
   }
   std::vector<long long> gpool_off(launches.size(), 0);
@@ -837,14 +875,17 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     const auto [variant, team, bytes, per_cta, first, count, Lmax] = launches[g];
     const int cap = wlg::main_batch_capacity(variant, team * per_cta, bytes * per_cta);
     if (cap <= 0) return fail(ex, WLG_ERR_CUDA, "main-run configuration does not fit an SM");
-    grids[g] = std::min(cap, (count + per_cta - 1) / per_cta);
+    const int ranks = wlg::variant_ranks(variant);
+    grids[g] = std::min(cap / ranks, (count + per_cta - 1) / per_cta) * ranks;
+    if (grids[g] == 0) return fail(ex, WLG_ERR_CUDA, "main-run configuration does not fit the device");
     if ((variant & wlg::kVariantGlobal) != 0 && !timed) {
       // a fixed arena or a budget may not hold a slice for every team that
       // the GPU could hold: fewer resident teams then take the problems in turn
       const long long slice = pool_slice(Lmax, team);
       const long long room = static_cast<long long>(ex.available(kGpool) / sizeof(double)) - gpool_doubles;
       const long long later = pool_later[g];
-      grids[g] = static_cast<int>(std::max(1LL, std::min<long long>(grids[g], (room - later) / (slice * per_cta))));
+      grids[g] = static_cast<int>(std::min<long long>(grids[g], (room - later) / (slice * per_cta)));
+      grids[g] = std::max(grids[g] / ranks, 1) * ranks;
       gpool_off[g] = gpool_doubles;
       gpool_doubles += grids[g] * per_cta * slice;
     }

@@ -99,8 +99,37 @@ __device__ __forceinline__ long long device_clock_ns()
   return t;
 }
 
-template <int kStore, bool kTight>
-__device__ void run_problem(const TeamHead& head, int p, const Team& team, int t, unsigned char* base, double* gslot,
+// A problem whose windows are spread over the CTAs of a thread-block cluster
+// (kCluster): every CTA runs its share as a team of its own.  Exchange between
+// its last window and the next CTA's first, a new energy and the convergence
+// votes go through distributed shared memory.
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_ranks()
+{
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// The address of p's counterpart in the shared memory of CTA `rank`.
+template <typename T>
+__device__ __forceinline__ T* at_rank(T* p, uint32_t rank)
+{
+  T* q;
+  asm volatile("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+  return q;
+}
+
+template <int kStore, bool kTight, bool kCluster>
+__device__ void run_problem(const TeamHead& head, int p, const Team& team, int t, unsigned char* base, double* gslot, long long gslot_doubles,
                             bool global_g, const uint32_t* __restrict__ Jpool, const uint32_t* __restrict__ latpool,
                             const int* __restrict__ winpool, const uint32_t* __restrict__ maskpool,
                             double* __restrict__ outpool, MainResult* __restrict__ results,
@@ -113,9 +142,9 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   const int P = team.size;
   // start time straight into the result slot: a value kept live through the
   // sweep costs the step registers
-  if (t == 0) results[p].t_start = device_clock_ns();
+  if (t == 0 && (!kCluster || cluster_rank() == 0)) results[p].t_start = device_clock_ns();
   // resumable run: state saved at the end of a launch, restored at the start
-  unsigned char* const st = d.off_state >= 0 ? statepool + d.off_state : nullptr;
+  unsigned char* const st = !kCluster && d.off_state >= 0 ? statepool + d.off_state : nullptr;
   const StateLayout& sl = head.state;
   const TeamLayout& lay = head.lay;
   // FP64 log g and the histogram change once per sweep: in the team's shared
@@ -147,8 +176,18 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   [[maybe_unused]] int* above = stab + 2 * d.I;
   int* win = reinterpret_cast<int*>(base + lay.off_win);  // start, end, base, Lb, E0
   int* misc = reinterpret_cast<int*>(base + lay.off_misc);
+  // this team's windows: b0 .. b0 + I - 1 of the problem's I_all
+  const int ranks = kCluster ? static_cast<int>(cluster_ranks()) : 1, rank = kCluster ? static_cast<int>(cluster_rank()) : 0;
+  const int I_all = d.I, W = d.W, b0 = kCluster ? I_all * rank / ranks : 0;
+  const int I = kCluster ? I_all * (rank + 1) / ranks - b0 : I_all;
+  const int t0 = b0 * W;  // the problem's index of this team's first walker
+  // where the team's CTAs meet, and the flags they share
+  auto sync_all = [&]() {
+    if constexpr (kCluster) cluster_sync();
+    else team.sync();
+  };
+  int* misc_all = kCluster ? at_rank(misc, 0) : misc;
   unsigned long long* new_key = reinterpret_cast<unsigned long long*>(misc + 4);
-  const int I = d.I, W = d.W;
   int* w_start = win;
   int* w_end = win + I;
   int* w_base = win + 2 * I;
@@ -157,7 +196,10 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   // ---- load the problem
   for (int q = t; q < d.nwM; q += P) mask[q] = maskpool[d.off_mask + q];
   for (int q = t; q < 2 * d.nwL; q += P) Js[q] = Jpool[d.off_J + q];
-  for (int q = t; q < 5 * I; q += P) win[q] = winpool[d.off_win + q];
+  for (int q = t; q < 5 * I; q += P) {
+    const int k = q / I;
+    win[q] = winpool[d.off_win + k * I_all + b0 + q - k * I];
+  }
   for (int q = t; q < I; q += P) {
     fwin[q] = kE;
     lnfw[q] = log(kE);
@@ -173,7 +215,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       H[c * P + t] = 0u;
     }
   if (t < 8) misc[t] = 0;
-  const bool live = t < d.nwalk;
+  const bool live = t < I * W;
   const int b = live ? t / W : 0;
   const int w = t - b * W;
   perm[t] = w;
@@ -239,7 +281,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   lt.stride = static_cast<uint32_t>(4 * P);
   lt.r = 0;
   if (live && !resumed) {
-    const uint32_t* src = latpool + d.off_lat + static_cast<long long>(b) * d.nwL;
+    const uint32_t* src = latpool + d.off_lat + static_cast<long long>(b0 + b) * d.nwL;
     if constexpr (kReg) {
       lt.r = src[0] | (d.nwL > 1 ? static_cast<uint64_t>(src[1]) << 32 : 0ull);
     } else if constexpr (kBonds) {
@@ -253,7 +295,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   int& E = wk.E;
   E = live ? win[4 * I + b] : 0;
   Stream& rng = wk.rng;
-  rng.init(d.key_wl, static_cast<uint64_t>(t), 0);
+  rng.init(d.key_wl, static_cast<uint64_t>(t0 + t), 0);
   const bool keys_differ = d.key_ex != static_cast<uint64_t>(d.key_wl);
   // what a factor exceeds: 2 the limit that resets a window (wl.cu:609), 1 the
   // loop's (mainrun.cu:243); kept per window, as factors rarely change (the
@@ -317,7 +359,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
   if (resumed && t == 0) misc[7] = static_cast<int>(outer + 1);  // finished windows get one averaging pass
   int launch_outer = 0;  // outer iterations of this launch
   bool suspended = false;
-  team.sync();
+  sync_all();
 
   for (;;) {
     if (d.max_outer > 0 && outer >= d.max_outer) {
@@ -332,9 +374,9 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       const double lnf = lnfw[b];  // log(f) (wl.cu:1124)
       auto log_g = [&](int c) { return G[c * P + t]; };
       auto new_energy = [&](int En, int step) {
-        misc[1] = 1;
+        misc_all[1] = 1;
         // reported: the last one found, by step, then by walker
-        atomicMax(new_key, static_cast<unsigned long long>(step) << 32 | static_cast<unsigned long long>(t) << 16 |
+        atomicMax(new_key, static_cast<unsigned long long>(step) << 32 | static_cast<unsigned long long>(t0 + t) << 16 |
                              static_cast<unsigned>(En + 32768));
       };
       // Fold the part's visits into histogram and log g, and with both at
@@ -408,9 +450,9 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       };
       wl_sweep<kStore, kTight, false>(common, wk, wmask, d.n_iter, frozen, lnf, exchange_next && ring_draws ? W : 0, log_g, is_bad, new_energy, fold);
     }
-    team.sync();
+    sync_all();
     ++outer;
-    if (misc[1] != 0) {
+    if (misc_all[1] != 0) {
       status = WLG_ERR_NEW_ENERGY;
       break;
     }
@@ -462,12 +504,12 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       chg[t] = 0;
       flat[t] = 0;
       if (cond[t] == 1 && stab[t] == 0) misc[7] = stamp + 1;
-      if (cond[t] != 1) misc[6] = stamp;
-      if ((over & 1) != 0) misc[2] = stamp;
+      if (cond[t] != 1) misc_all[6] = stamp;
+      if ((over & 1) != 0) misc_all[2] = stamp;
     }
-    team.sync();
-    const bool done = misc[6] != stamp;
-    const bool stop = misc[2] != stamp;  // the largest factor is at the limit
+    sync_all();
+    const bool done = misc_all[6] != stamp;
+    const bool stop = misc_all[2] != stamp;  // the largest factor is at the limit
     // ---- replica exchange (wl.cu:785-890)
     if (!done && exchange_next) {
       if (live) {
@@ -477,7 +519,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
           lat_s[P + t] = static_cast<uint32_t>(lt.r >> 32);
         }
         if (keys_differ) {
-          rng.init(d.key_ex, static_cast<uint64_t>(t), rng.pos);
+          rng.init(d.key_ex, static_cast<uint64_t>(t0 + t), rng.pos);
         } else if (!ring_draws) {
           rng.refill();
         }
@@ -485,9 +527,9 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       const int nw = kReg ? 2 : d.nwL;
       for (int pass = 0; pass < 2; ++pass) {
         const int even = pass == 0;
-        team.sync();
-        const int par = (b + d.parity_base) & 1;
-        const bool active = live && b < I - 1 && ((even && par == 0) || (!even && par == 1));
+        sync_all();
+        const int par = (b0 + b + d.parity_base) & 1;
+        const bool active = live && b0 + b < I_all - 1 && ((even && par == 0) || (!even && par == 1));
         if (active && w == 0) {  // Fisher-Yates by the window's first walker
           for (int i = W - 1; i > 0; --i) {
             // trunc(u (i + 0.999999)), as the sweep's site among i + 1
@@ -501,17 +543,35 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
         }
         team.sync();
         if (active) {
-          const int o = (b + 1) * W + perm[t];
-          const int et = E_s[t], eo = E_s[o];
-          if (et >= w_start[b + 1] && et <= w_end[b + 1] && eo >= w_start[b] && eo <= w_end[b]) {
-            const int nb = w_base[b + 1];
+          // the partner's window: the next one, or the next CTA's first
+          int o = (b + 1) * W + perm[t], next = b + 1, I_next = I;
+          int *E_o = E_s, *win_o = win;
+          uint32_t* lat_o = lat_s;
+          const double* G_o = G;
+          if (kCluster && next == I) {
+            o = perm[t];
+            next = 0;
+            I_next = I_all * (rank + 2) / ranks - I_all * (rank + 1) / ranks;
+            E_o = at_rank(E_s, rank + 1);
+            win_o = at_rank(win, rank + 1);
+            lat_o = at_rank(lat_s, rank + 1);
+            G_o = global_g ? G + gslot_doubles : at_rank(G, rank + 1);
+          }
+          const int et = E_s[t], eo = E_o[o];
+          if (et >= win_o[next] && et <= win_o[I_next + next] && eo >= lo && eo <= hi) {
+            const int nb = win_o[2 * I_next + next];
             const double gi_x = G[((et - bb) >> d.lg) * P + t];
             const double gi_y = G[((eo - bb) >> d.lg) * P + t];
-            const double gj_y = G[((eo - nb) >> d.lg) * P + o];
-            const double gj_x = G[((et - nb) >> d.lg) * P + o];
+            // another CTA's log g in global memory: past this SM's L1
+            const auto g_o = [&](int e) {
+              const double* a = G_o + ((e - nb) >> d.lg) * P + o;
+              return kCluster && global_g ? __ldcg(a) : *a;
+            };
+            const double gj_y = g_o(eo);
+            const double gj_x = g_o(et);
             if (exchange_accepts(draw(), gi_x - gi_y, gj_y - gj_x)) {
               E_s[t] = eo;
-              E_s[o] = et;
+              E_o[o] = et;
               // four words at a time: their loads overlap
               for (int q = 0; q < nw; q += 4) {
                 uint32_t a[4], c[4];
@@ -519,24 +579,24 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
                 for (int u = 0; u < 4; ++u) {
                   const int r = min(q + u, nw - 1) * P;
                   a[u] = lat_s[r + t];
-                  c[u] = lat_s[r + o];
+                  c[u] = lat_o[r + o];
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                   const int r = min(q + u, nw - 1) * P;
                   lat_s[r + t] = c[u];
-                  lat_s[r + o] = a[u];
+                  lat_o[r + o] = a[u];
                 }
               }
             }
           }
         }
       }
-      team.sync();
+      sync_all();
       if (live) {
         E = E_s[t];
         if constexpr (kReg) lt.r = lat_s[t] | static_cast<uint64_t>(lat_s[P + t]) << 32;
-        if (keys_differ) rng.init(d.key_wl, static_cast<uint64_t>(t), rng.pos);
+        if (keys_differ) rng.init(d.key_wl, static_cast<uint64_t>(t0 + t), rng.pos);
       }
     }
     if (d.exch_mode == 1) ++counter;
@@ -596,12 +656,17 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
 
   // ---- results
   if (live && w == 0) {
-    for (int c = 0; c < d.L; ++c) outpool[d.off_out + static_cast<long long>(b) * d.L + c] = G[c * P + t];
+    for (int c = 0; c < d.L; ++c) outpool[d.off_out + static_cast<long long>(b0 + b) * d.L + c] = G[c * P + t];
   }
-  if (t == 0) {
+  if (rank == 0 && t == 0) {
     MainResult r{};
     r.status = status;
-    r.new_energy = misc[1] != 0 ? static_cast<int>(*new_key & 0xFFFFu) - 32768 : 0;
+    if (status == WLG_ERR_NEW_ENERGY) {
+      unsigned long long key = *new_key;
+      if constexpr (kCluster)
+        for (int q = 1; q < ranks; ++q) key = max(key, *at_rank(new_key, q));
+      r.new_energy = static_cast<int>(key & 0xFFFFu) - 32768;
+    }
     r.outer = outer;
     r.flips = outer * static_cast<long long>(d.nwalk) * d.n_iter;
     r.done = 1;
@@ -609,10 +674,10 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
     r.t_end = device_clock_ns();
     results[p] = r;
   }
-  team.sync();
+  sync_all();  // no CTA leaves or starts anew while another may still reach into it
 }
 
-template <int kStore, bool kTight, int kMaxThreads>
+template <int kStore, bool kTight, bool kCluster, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads)
   k_main_batch(const MainDesc* __restrict__ descs, const int* __restrict__ order, int n, int team_size, int team_bytes,
                int global_g, int* __restrict__ next, double* __restrict__ gpool, long long gslot_doubles,
@@ -630,10 +695,18 @@ __global__ void __launch_bounds__(kMaxThreads)
   TeamHead own;
   TeamHead* head = kTight ? &own : reinterpret_cast<TeamHead*>(base);
   for (;;) {
-    if (t == 0) *slot = atomicAdd(next, 1);
-    team.sync();
-    const int q = *slot;
-    team.sync();
+    int q;
+    if constexpr (kCluster) {  // one problem per cluster, taken by its first CTA
+      if (t == 0 && cluster_rank() == 0) *slot = atomicAdd(next, 1);
+      cluster_sync();
+      q = *at_rank(slot, 0);
+      cluster_sync();
+    } else {
+      if (t == 0) *slot = atomicAdd(next, 1);
+      team.sync();
+      q = *slot;
+      team.sync();
+    }
     if (q >= n) return;
     const int p = order[q];
     if (descs[p].off_state >= 0 && results[p].done != 0) continue;  // resumable run that finished in an earlier launch
@@ -648,7 +721,7 @@ __global__ void __launch_bounds__(kMaxThreads)
     double* gslot = global_g != 0 && gpool != nullptr
                       ? gpool + (static_cast<long long>(blockIdx.x) * (blockDim.x / team_size) + tix) * gslot_doubles
                       : nullptr;
-    run_problem<kStore, kTight>(*head, p, team, t, base, gslot, global_g != 0, Jpool, latpool, winpool, maskpool, outpool,
+    run_problem<kStore, kTight, kCluster>(*head, p, team, t, base, gslot, gslot_doubles, global_g != 0, Jpool, latpool, winpool, maskpool, outpool,
                                 results, statepool);
   }
 }
@@ -657,15 +730,28 @@ __global__ void __launch_bounds__(kMaxThreads)
 template <int kMaxThreads>
 MainFn main_fn_of(int store, bool tight)
 {
+#define WLG_MAIN_FN(S) \
+  (tight ? &k_main_batch<S, true, false, kMaxThreads> : &k_main_batch<S, false, false, kMaxThreads>)
   switch (store) {
-    case kStoreReg: return tight ? &k_main_batch<kStoreReg, true, kMaxThreads> : &k_main_batch<kStoreReg, false, kMaxThreads>;
-    case kStoreTable:
-      return tight ? &k_main_batch<kStoreTable, true, kMaxThreads> : &k_main_batch<kStoreTable, false, kMaxThreads>;
-    case kStoreRows:
-      return tight ? &k_main_batch<kStoreRows, true, kMaxThreads> : &k_main_batch<kStoreRows, false, kMaxThreads>;
-    case kStoreBonds: return &k_main_batch<kStoreBonds, false, kMaxThreads>;
-    default:
-      return tight ? &k_main_batch<kStoreLinear, true, kMaxThreads> : &k_main_batch<kStoreLinear, false, kMaxThreads>;
+    case kStoreReg: return WLG_MAIN_FN(kStoreReg);
+    case kStoreTable: return WLG_MAIN_FN(kStoreTable);
+    case kStoreRows: return WLG_MAIN_FN(kStoreRows);
+    case kStoreBonds: return &k_main_batch<kStoreBonds, false, false, kMaxThreads>;
+    default: return WLG_MAIN_FN(kStoreLinear);
+  }
+#undef WLG_MAIN_FN
+}
+
+// The kernel for problems spread over a cluster.
+template <int kMaxThreads>
+MainFn main_fn_cluster_of(int store)
+{
+  switch (store) {
+    case kStoreReg: return &k_main_batch<kStoreReg, false, true, kMaxThreads>;
+    case kStoreTable: return &k_main_batch<kStoreTable, false, true, kMaxThreads>;
+    case kStoreRows: return &k_main_batch<kStoreRows, false, true, kMaxThreads>;
+    case kStoreBonds: return &k_main_batch<kStoreBonds, false, true, kMaxThreads>;
+    default: return &k_main_batch<kStoreLinear, false, true, kMaxThreads>;
   }
 }
 

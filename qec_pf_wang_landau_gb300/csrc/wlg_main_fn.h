@@ -1,5 +1,6 @@
 // Entry points of the persistent main-run kernel, one translation unit per
-// largest CTA size (wlg_main_256.cu, wlg_main_512.cu, wlg_main_1024.cu).
+// largest CTA size (wlg_main_256.cu, wlg_main_512.cu, wlg_main_1024.cu), and one
+// for clusters (wlg_main_cluster.cu).
 #pragma once
 
 #include <cstdint>
@@ -15,5 +16,6 @@ using MainFn = void (*)(const MainDesc*, const int*, int, int, int, int, int*, d
 MainFn main_fn_256(int store, bool tight);
 MainFn main_fn_512(int store, bool tight);
 MainFn main_fn_1024(int store, bool tight);
+MainFn main_fn_cluster(int store);  // a problem's windows spread over a cluster
 
 }  // namespace wlg

@@ -23,6 +23,15 @@ CASES = {
     "tight_rows": (16, 16, 0, 0.10, "c", 4242, 1, 128, 128, 25600, 64, 12, 0.3, 0.8, 1e-8, 130, 1, 1, 0, 2),
     "tight_table": (8, 8, 1, 0.10, "v", 16, 1, 128, 64, 12800, 32, 32, 0.28, 0.8, 1e-3, 130, 1, 1, 0, 2),
     "tight_linear": (2, 40, 0, 0.10, "v", 17, 1, 128, 64, 16000, 32, 32, 0.15, 0.8, 1e-3, 130, 1, 1, 0, 2),
+    # windows spread over clusters of 2, 4 and 8 CTAs, evenly and not, in every lattice storage;
+    # exchange crosses CTAs, its draws come from the ring or (W = 16) not
+    "cluster_table": (8, 8, 0, 0.10, "v", 21, 1, 128, 64, 6400, 11, 30, 0.28, 0.8, 1e-3, 200, 1, 1, 0, 8),
+    "cluster_reg": (2, 30, 1, 0.10, "v", 22, 1, 128, 32, 9000, 10, 26, 0.28, 0.8, 1e-3, 200, 1, 1, 1, 8),
+    "cluster_bonds": (12, 12, 1, 0.10, "c", 23, 1, 128, 64, 14400, 32, 16, 0.3, 0.8, 1e-3, 150, 1, 1, 0, 6),
+    "cluster_rows": (20, 20, 0, 0.10, "h", 24, 1, 128, 128, 40000, 43, 12, 0.3, 0.8, 1e-3, 120, 2, 1, 0, 4),
+    "cluster_linear": (3, 40, 0, 0.10, "i", 25, 1, 128, 64, 12000, 13, 20, 0.28, 0.8, 1e-3, 150, 1, 1, 0, 6),
+    "cluster_8": (10, 10, 0, 0.10, "v", 26, 1, 128, 64, 10000, 30, 34, 0.28, 0.8, 1e-3, 100, 1, 1, 0, 4),
+    "cluster_global": (20, 20, 0, 0.10, "v", 27, 1, 128, 64, 40000, 16, 16, 0.28, 0.8, 1e-3, 100, 1, 1, 0, 3),
     # one step, less than a chunk, a chunk and one step; more than a part
     "steps_1": (6, 6, 0, 0.04, "i", 18, 1, 128, 32, 2000, 4, 3, 0.25, 0.8, 1e-3, 1, 3, 1, 0, 200),
     "steps_7": (6, 6, 1, 0.04, "i", 18, 1, 128, 32, 2000, 4, 3, 0.25, 0.8, 1e-3, 7, 3, 1, 0, 60),
