@@ -226,10 +226,17 @@ inline int admission_bytes(const MainDesc& d, int team)
 
 // The kernel of d: everything in shared memory where it fits, else log g and
 // the histogram in global memory (read and written once per sweep), else the
-// tight layout.  Problems of one launch share it.
-inline int kernel_variant(const MainDesc& d, int team)
+// tight layout.  Rows of 17 to 32 sites keep their bonds in two words where that
+// fits (24x24, 128 walkers on an SM: 0.25 -> 0.19 us a step against rows), not in
+// resumable runs, whose saved lattices have a word a row.  Problems of one launch
+// share it.
+inline int kernel_variant(const MainDesc& d, int team, bool resumable)
 {
   const int store = lattice_store(d, false);
+  if (store == kStoreRows && !resumable) {
+    if (team_bytes(d, kStoreBonds2, team) <= kSmemBytes) return kStoreBonds2;
+    if (team_bytes(d, kStoreBonds2 | kVariantGlobal, team) <= kSmemBytes) return kStoreBonds2 | kVariantGlobal;
+  }
   if (team_bytes(d, store, team) <= kSmemBytes) return store;
   if (team_bytes(d, store | kVariantGlobal, team) <= kSmemBytes) return store | kVariantGlobal;
   return tight_variant(d);

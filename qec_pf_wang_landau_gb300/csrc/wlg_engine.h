@@ -181,8 +181,8 @@ WLG_HD inline StateLayout state_layout(int P, int I, int nwL, int L)
 // register (N <= 64), the register with a neighbour table (X, Y >= 3), or one
 // row per shared word (lattice_rows).  Bonds: for rows of up to 16 sites, the
 // unsatisfied right bonds (low half) and down bonds (high half) of a row in one
-// word instead of its spins.
-enum Store { kStoreLinear = 0, kStoreReg = 1, kStoreTable = 2, kStoreRows = 3, kStoreBonds = 4 };
+// word instead of its spins; for rows of up to 32, in two words.
+enum Store { kStoreLinear = 0, kStoreReg = 1, kStoreTable = 2, kStoreRows = 3, kStoreBonds = 4, kStoreBonds2 = 5 };
 
 // Draws a walker keeps ahead (a power of two), and the bytes of a warp's ring
 // of them: slot after slot of 32 lanes, the first slot repeated at the end.
@@ -230,7 +230,7 @@ WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, boo
   t.off_ring = o;
   o = align16(o + (tight ? 0 : team / 32 * kRingWarpBytes));
   t.off_lat = o;  // the lattice, or the exchange staging of a register lattice
-  o = align16(o + 4 * (reg ? 2 : d.nwL) * team);
+  o = align16(o + 4 * (reg ? 2 : (store == kStoreBonds2 ? 2 * d.nwL : d.nwL)) * team);
   t.off_E = o;
   o = align16(o + 4 * team);
   t.off_perm = o;
@@ -240,7 +240,7 @@ WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, boo
   t.off_J = o;
   o = align16(o + 4 * 2 * d.nwL);
   t.off_tab = o;  // neighbour table and degrees per site, or bond masks per column and per row
-  o = align16(o + (store == kStoreTable ? 20 * d.N : (store == kStoreBonds ? align16(8 * d.Y) + 16 * d.X : 0)));
+  o = align16(o + (store == kStoreTable ? 20 * d.N : (store >= kStoreBonds ? align16(8 * d.Y) + 16 * d.X : 0)));
   t.off_f = o;  // f [I], then ln f [I]
   o = align16(o + 16 * I);
   t.off_cond = o;

@@ -778,15 +778,16 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex.device);
   // one launch per (form, team size); the form by lattice storage (fit_form)
   std::map<std::pair<int, int>, std::vector<int>> groups;
-  const int spread = time_limit_s > 0 ? 1 : spread_ranks(prep, sms);
+  const bool resumable = time_limit_s > 0;
+  const int spread = resumable ? 1 : spread_ranks(prep, sms);
   for (int i = 0; i < m; ++i) {
     const MainDesc& d = prep.main[i];
     const int ranks = problem_ranks(d, spread), team = rank_team(d, ranks);
-    const int variant = wlg::kernel_variant(d, team);
+    const int variant = wlg::kernel_variant(d, team, resumable);
     if (ranks > 1 && (variant & wlg::kVariantTight) == 0) {
       groups[{variant | ranks * wlg::kVariantRanks, team}].push_back(i);
     } else {
-      groups[{wlg::kernel_variant(d, d.team), d.team}].push_back(i);
+      groups[{wlg::kernel_variant(d, d.team, resumable), d.team}].push_back(i);
     }
   }
   // Longest problems first (larger lattices take more outer iterations of
@@ -1388,7 +1389,7 @@ wlg_status wlg_context_autotune(wlg_context* ctx, const wlg_problem* problems, i
     std::map<std::pair<int, int>, std::vector<int>> groups;
     for (size_t i = 0; i < prep.main.size(); ++i) {
       const MainDesc& d = prep.main[i];
-      groups[{kernel_variant(d, d.team), d.team}].push_back(static_cast<int>(i));
+      groups[{kernel_variant(d, d.team, false), d.team}].push_back(static_cast<int>(i));
     }
     std::map<std::pair<int, int>, int> best;
     std::vector<wlg_tuning> found;

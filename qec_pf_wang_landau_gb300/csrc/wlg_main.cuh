@@ -137,7 +137,8 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
 {
   constexpr bool kTable = kStore == kStoreTable;
   constexpr bool kReg = kStore == kStoreReg || kTable;
-  constexpr bool kBonds = kStore == kStoreBonds;
+  constexpr bool kTwo = kStore == kStoreBonds2;
+  constexpr bool kBonds = kStore == kStoreBonds || kTwo;
   const MainDesc& d = head.d;
   const int P = team.size;
   // start time straight into the result slot: a value kept live through the
@@ -272,7 +273,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
     }
   }
   if constexpr (kBonds) {
-    fill_bond_tables(reinterpret_cast<uint2*>(base + lay.off_tab),
+    fill_bond_tables<kTwo>(reinterpret_cast<uint2*>(base + lay.off_tab),
                      reinterpret_cast<uint4*>(base + lay.off_tab + align16(8 * d.Y)), d.X, d.Y, open_bc, dlt_bytes, t, P);
   }
   Walker<kTight> wk;
@@ -286,8 +287,16 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       lt.r = src[0] | (d.nwL > 1 ? static_cast<uint64_t>(src[1]) << 32 : 0ull);
     } else if constexpr (kBonds) {
       // unsatisfied bonds of the start lattice
-      for (int i = 0; i < d.X; ++i)
-        lat_s[i * P + t] = bond_word(src[i], src[i + 1 < d.X ? i + 1 : 0], Jr_s[i], Jd_s[i], d.Y, open_bc, i + 1 == d.X);
+      for (int i = 0; i < d.X; ++i) {
+        uint32_t h, v;
+        bond_bits(src[i], src[i + 1 < d.X ? i + 1 : 0], Jr_s[i], Jd_s[i], d.Y, open_bc, i + 1 == d.X, h, v);
+        if constexpr (kTwo) {
+          lat_s[2 * i * P + t] = h;
+          lat_s[(2 * i + 1) * P + t] = v;
+        } else {
+          lat_s[i * P + t] = h | v << 16;
+        }
+      }
     } else {
       for (int q = 0; q < d.nwL; ++q) lat_s[q * P + t] = src[q];
     }
@@ -524,7 +533,7 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
           rng.refill();
         }
       }
-      const int nw = kReg ? 2 : d.nwL;
+      const int nw = kReg ? 2 : (kTwo ? 2 * d.nwL : d.nwL);
       for (int pass = 0; pass < 2; ++pass) {
         const int even = pass == 0;
         sync_all();
@@ -737,6 +746,7 @@ MainFn main_fn_of(int store, bool tight)
     case kStoreTable: return WLG_MAIN_FN(kStoreTable);
     case kStoreRows: return WLG_MAIN_FN(kStoreRows);
     case kStoreBonds: return &k_main_batch<kStoreBonds, false, false, kMaxThreads>;
+    case kStoreBonds2: return &k_main_batch<kStoreBonds2, false, false, kMaxThreads>;
     default: return WLG_MAIN_FN(kStoreLinear);
   }
 #undef WLG_MAIN_FN
@@ -751,6 +761,7 @@ MainFn main_fn_cluster_of(int store)
     case kStoreTable: return &k_main_batch<kStoreTable, false, true, kMaxThreads>;
     case kStoreRows: return &k_main_batch<kStoreRows, false, true, kMaxThreads>;
     case kStoreBonds: return &k_main_batch<kStoreBonds, false, true, kMaxThreads>;
+    case kStoreBonds2: return &k_main_batch<kStoreBonds2, false, true, kMaxThreads>;
     default: return &k_main_batch<kStoreLinear, false, true, kMaxThreads>;
   }
 }

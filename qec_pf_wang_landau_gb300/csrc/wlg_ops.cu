@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
     Jr[q] = bits;
   }
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_tab);
-  fill_bond_tables(col, reinterpret_cast<uint4*>(smem + l.off_tab + align16(8 * Y)), X, Y, open, 2 * (256 >> lg), lane, 32);
+  fill_bond_tables<false>(col, reinterpret_cast<uint4*>(smem + l.off_tab + align16(8 * Y)), X, Y, open, 2 * (256 >> lg), lane, 32);
   __syncwarp();
   const int b = t / (a.wpi / a.n_int);
   const int e_first = a.start[k * a.n_int], e_last = a.end[k * a.n_int + a.n_int - 1];

@@ -634,7 +634,7 @@ void wlg_server::finish_admission(AdmitJob& aj)
     }
     MainDesc d = prep.main[main_of[k]];
     const BlockLayout bl = block_layout(d.team, d.I, d.L, d.nwL, d.nwM);
-    const int form = kernel_variant(d, d.team);
+    const int form = kernel_variant(d, d.team, true);
     if (admission_bytes(d, d.team) > kSmemLimit || bl.bytes > bb.bytes) {
       arena.release(boff, bb.bytes);
       class_done(id, cls, WLG_ERR_INVALID, 0, {});

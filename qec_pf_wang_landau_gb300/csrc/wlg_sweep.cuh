@@ -297,7 +297,9 @@ __device__ __forceinline__ uint32_t shared_addr(const void* p)
 // Bond tables: per column the bits of its two horizontal bonds (low half) and
 // its down bond (high half), and its missing bonds in bin bytes; per row the
 // masks of what exists in its own word and in the word above, and its missing
-// bonds.
+// bonds.  kTwo: horizontal bonds alone per column, masks of all or nothing for
+// the down bonds of the row and of the one above.
+template <bool kTwo>
 __device__ __forceinline__ void fill_bond_tables(uint2* col, uint4* row, int X, int Y, bool open, int dlt_bytes, int t,
                                                  int P)
 {
@@ -305,27 +307,37 @@ __device__ __forceinline__ void fill_bond_tables(uint2* col, uint4* row, int X, 
     uint32_t h = (1u << j) | (1u << (j == 0 ? Y - 1 : j - 1));
     if (open) h &= ~(1u << (Y - 1));
     const int miss = open ? (j == 0 ? 1 : 0) + (j == Y - 1 ? 1 : 0) : 0;
-    col[j] = make_uint2(h | 0x10000u << j, static_cast<uint32_t>(-miss * dlt_bytes));
+    col[j] = make_uint2(kTwo ? h : h | 0x10000u << j, static_cast<uint32_t>(-miss * dlt_bytes));
   }
   for (int i = t; i < X; i += P) {
     const bool up = !open || i > 0, dn = !open || i < X - 1;
     const int miss = (up ? 0 : 1) + (dn ? 0 : 1);
-    row[i] = make_uint4(dn ? 0xFFFFFFFFu : 0x0000FFFFu, up ? 0xFFFF0000u : 0u, static_cast<uint32_t>(-miss * dlt_bytes), 0u);
+    row[i] = make_uint4(dn ? 0xFFFFFFFFu : (kTwo ? 0u : 0x0000FFFFu), up ? (kTwo ? 0xFFFFFFFFu : 0xFFFF0000u) : 0u,
+                        static_cast<uint32_t>(-miss * dlt_bytes), 0u);
   }
 }
 
-// The bond word of a row from its spin bits r, those of the row below and the
-// coupling bits: bit j is bond (i, j)-(i, j + 1), bit 16 + j bond (i, j)-(i + 1, j);
-// set when unsatisfied, 0 when missing.
-__device__ __forceinline__ uint32_t bond_word(uint32_t r, uint32_t below, uint32_t Jr, uint32_t Jd, int Y, bool open,
-                                              bool last)
+// The bonds of a row from its spin bits r, those of the row below and the
+// coupling bits: bit j of h is bond (i, j)-(i, j + 1), bit j of v bond
+// (i, j)-(i + 1, j); set when unsatisfied, 0 when missing.
+__device__ __forceinline__ void bond_bits(uint32_t r, uint32_t below, uint32_t Jr, uint32_t Jd, int Y, bool open, bool last,
+                                          uint32_t& h, uint32_t& v)
 {
-  const uint32_t all = (1u << Y) - 1u;
-  uint32_t h = (r ^ ((r >> 1) | ((r & 1u) << (Y - 1))) ^ Jr) & all, v = (r ^ below ^ Jd) & all;
+  const uint32_t all = Y == 32 ? 0xFFFFFFFFu : (1u << Y) - 1u;
+  h = (r ^ ((r >> 1) | ((r & 1u) << (Y - 1))) ^ Jr) & all;
+  v = (r ^ below ^ Jd) & all;
   if (open) {
     h &= ~(1u << (Y - 1));
     if (last) v = 0;
   }
+}
+
+// Both in one word, rows of up to 16 sites.
+__device__ __forceinline__ uint32_t bond_word(uint32_t r, uint32_t below, uint32_t Jr, uint32_t Jd, int Y, bool open,
+                                              bool last)
+{
+  uint32_t h, v;
+  bond_bits(r, below, Jr, Jd, Y, open, last, h, v);
   return h | v << 16;
 }
 
@@ -387,7 +399,8 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
   constexpr bool kTable = kStore == kStoreTable;
   constexpr bool kReg = kStore == kStoreReg || kTable;
   constexpr bool kRows = kStore == kStoreRows;
-  constexpr bool kBonds = kStore == kStoreBonds;
+  constexpr bool kTwo = kStore == kStoreBonds2;
+  constexpr bool kBonds = kStore == kStoreBonds || kTwo;
   // Pairs of steps unrolled in the persistent run, so that ptxas schedules
   // across them: 16x16 on every SM 0.368 -> 0.339 us a step, 12x12 0.157 ->
   // 0.148, 6x6 0.129 -> 0.122.  Not for the longer steps of rows and linear
@@ -574,7 +587,7 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
     auto step = [&](auto beside1, auto beside2) {
       uint32_t next;           // address (tight: index) of the proposal's bin
       [[maybe_unused]] uint64_t flip_mask = 0;  // register spins
-      [[maybe_unused]] uint32_t wa = 0, wb = 0, na = 0, nb = 0;  // shared words to rewrite on acceptance
+      [[maybe_unused]] uint32_t wa = 0, wb = 0, wc = 0, na = 0, nb = 0, nc = 0;  // shared words to rewrite on acceptance
       [[maybe_unused]] int dE = 0;
       if constexpr (kTable) {
         const int deg = static_cast<int>(cs.col.x);
@@ -585,14 +598,29 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
         if constexpr (kTight) dE = sgn * 2 * (deg / dlt_bytes - 2 * unsat);
         else next = (cur + sgn * deg) + unsat * (-2 * dlt_bytes * sgn);
       } else if constexpr (kBonds) {
-        wa = lt.a + cs.i * lt.stride;
-        wb = lt.a + min(cs.i - 1u, uX - 1u) * lt.stride;
-        na = lds_u32(wa);
-        nb = lds_u32(wb);
-        const uint32_t m1 = cs.col.x & cs.row.x, m2 = cs.col.x & cs.row.y;
-        const int unsat = __popc(na & m1) + __popc(nb & m2);
-        na ^= m1;
-        nb ^= m2;
+        int unsat;
+        if constexpr (kTwo) {
+          wa = lt.a + 2u * cs.i * lt.stride;
+          wc = wa + lt.stride;
+          wb = lt.a + (2u * min(cs.i - 1u, uX - 1u) + 1u) * lt.stride;
+          na = lds_u32(wa);
+          nb = lds_u32(wb);
+          nc = lds_u32(wc);
+          const uint32_t m = 1u << cs.j, m2 = m & cs.row.y, m3 = m & cs.row.x;
+          unsat = __popc(na & cs.col.x) + __popc(nb & m2) + __popc(nc & m3);
+          na ^= cs.col.x;
+          nb ^= m2;
+          nc ^= m3;
+        } else {
+          wa = lt.a + cs.i * lt.stride;
+          wb = lt.a + min(cs.i - 1u, uX - 1u) * lt.stride;
+          na = lds_u32(wa);
+          nb = lds_u32(wb);
+          const uint32_t m1 = cs.col.x & cs.row.x, m2 = cs.col.x & cs.row.y;
+          unsat = __popc(na & m1) + __popc(nb & m2);
+          na ^= m1;
+          nb ^= m2;
+        }
         next = (cur + 4 * dlt_bytes + cs.col.y + cs.row.z) + unsat * (-2 * dlt_bytes);
       } else {
         if constexpr (kRows) {
@@ -653,6 +681,7 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
       } else {
         sts_if(acc, wa, na);
         if constexpr (kBonds) sts_if(acc, wb, nb);
+        if constexpr (kTwo) sts_if(acc, wc, nc);
       }
       if constexpr (kSign) wk.s0 ^= acc & ((cs.i | cs.j) == 0) ? 1u : 0u;
       cur = acc ? next : cur;
@@ -673,18 +702,33 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
         const int i = static_cast<int>((static_cast<uint32_t>(site) * d.site_magic) >> 20), j = site - i * d.Y;
         const int c_cur = kTight ? static_cast<int>(cur) : static_cast<int>((cur - bin0) / bin_bytes);
         uint32_t w1 = 0, w2 = 0, n1 = 0, n2 = 0;
+        [[maybe_unused]] uint32_t w3 = 0, n3 = 0;
         int dE;
         if constexpr (kBonds) {
-          w1 = lt.a + static_cast<uint32_t>(i) * lt.stride;
-          w2 = lt.a + static_cast<uint32_t>(i == 0 ? d.X - 1 : i - 1) * lt.stride;
+          const uint32_t iu = static_cast<uint32_t>(i == 0 ? d.X - 1 : i - 1);
           const uint2 cm = lds_u64(jt_a + 8 * j);
           const uint4 rm = lds_u128(rt_a + 16 * i);
-          const uint32_t m1 = cm.x & rm.x, m2 = cm.x & rm.y;
+          uint32_t m1, m2, m3 = 0;
+          if constexpr (kTwo) {
+            w1 = lt.a + 2u * static_cast<uint32_t>(i) * lt.stride;
+            w3 = w1 + lt.stride;
+            w2 = lt.a + (2u * iu + 1u) * lt.stride;
+            m1 = cm.x;
+            m2 = (1u << j) & rm.y;
+            m3 = (1u << j) & rm.x;
+            n3 = lds_u32(w3);
+          } else {
+            w1 = lt.a + static_cast<uint32_t>(i) * lt.stride;
+            w2 = lt.a + iu * lt.stride;
+            m1 = cm.x & rm.x;
+            m2 = cm.x & rm.y;
+          }
           n1 = lds_u32(w1);
           n2 = lds_u32(w2);
-          dE = 2 * (__popc(m1) + __popc(m2) - 2 * (__popc(n1 & m1) + __popc(n2 & m2)));
+          dE = 2 * (__popc(m1) + __popc(m2) + __popc(m3) - 2 * (__popc(n1 & m1) + __popc(n2 & m2) + __popc(n3 & m3)));
           n1 ^= m1;
           n2 ^= m2;
+          n3 ^= m3;
         } else if constexpr (kRows) {
           dE = flip_energy_rows(lt, Jr_s, Jd_s, i, j, d, hedge, open_bc, w1, n1);
         } else {
@@ -716,6 +760,7 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
               } else {
                 sts_if(true, w1, n1);
                 if constexpr (kBonds) sts_if(true, w2, n2);
+                if constexpr (kTwo) sts_if(true, w3, n3);
               }
               if (c_new != c_cur) {
                 a_c = lds_pair(bin0 + c_new * bin_bytes).x;

@@ -11,13 +11,14 @@ pytestmark = pytest.mark.gpu
 
 #  X, Y, boundary, prob, cls, seed, R, pre_w, pre_i, pre_n, I, W, overlap, alpha, beta, n_iter, xc, xmode, gpar, outer
 CASES = {
-    # 65-site and longer lattices: rows of 2, 16 (bonds), 17, 32 (rows) and 33 sites (linear words)
+    # 65-site and longer lattices: rows of 2, 16 (bonds), 17, 32 (two-word bonds) and 33 sites (linear words)
     "bonds_40x2": (40, 2, 0, 0.10, "v", 11, 1, 64, 32, 8000, 6, 3, 0.25, 0.8, 1e-3, 300, 2, 1, 0, 6),
     "bonds_40x2_open": (40, 2, 1, 0.10, "h", 11, 1, 64, 32, 8000, 6, 3, 0.25, 0.8, 1e-3, 300, 2, 1, 0, 6),
     "bonds_5x16_open": (5, 16, 1, 0.10, "c", 12, 1, 64, 32, 8000, 6, 4, 0.25, 0.8, 1e-3, 300, 1, 1, 0, 6),
     "rows_5x17": (5, 17, 0, 0.10, "c", 13, 1, 64, 32, 8500, 6, 4, 0.25, 0.8, 1e-3, 300, 1, 1, 0, 6),
     "rows_5x17_open": (5, 17, 1, 0.10, "i", 13, 1, 64, 32, 8500, 6, 4, 0.25, 0.8, 1e-3, 300, 1, 1, 0, 6),
     "rows_3x32": (3, 32, 0, 0.10, "v", 14, 1, 64, 32, 9600, 6, 4, 0.25, 0.8, 1e-3, 300, 1, 1, 0, 6),
+    "rows_24x24": (24, 24, 0, 0.10, "c", 28, 1, 128, 64, 57600, 64, 8, 0.3, 0.8, 1e-8, 60, 1, 1, 0, 2),
     "linear_3x33": (3, 33, 0, 0.10, "v", 15, 1, 64, 32, 9900, 6, 4, 0.25, 0.8, 1e-3, 300, 1, 1, 0, 6),
     # states whose guard bins and draw ring do not fit: 1024 walkers
     "tight_rows": (16, 16, 0, 0.10, "c", 4242, 1, 128, 128, 25600, 64, 12, 0.3, 0.8, 1e-8, 130, 1, 1, 0, 2),
@@ -57,3 +58,28 @@ def test_main_run_edges_bit_exact(cuda, name):
         o = ref["off_hist"][b * W]
         want = ref["logG"][o:o + (e[b] - s[b] + 1)]
         assert np.array_equal(wins[b], want), f"window {b}: max |d| {np.abs(wins[b] - want).max()}"
+
+
+@pytest.mark.parametrize("X,Y,boundary", [(5, 17, 0), (5, 17, 1), (4, 32, 0), (9, 9, 1), (3, 33, 0)])
+def test_resumable_main_run_equals_the_uninterrupted_one(cuda, X, Y, boundary):
+    """Under a time limit the main run saves its state every few iterations, and
+    lattices stay in the saved form's storage: the same curves as without."""
+    import ctypes as C
+    import qec_pf_wang_landau_gb300 as wlg
+    N = X * Y
+    p = wlg.problem(X, Y, boundary=boundary, prob=0.08, error_class="v", seed=31, pre_walkers=64, pre_intervals=24,
+                    pre_iterations=100 * N, intervals=6, walkers_per_interval=3, beta=0.3, iterations=400,
+                    exchange_every=1)
+    ctx = wlg.Context(0)
+    (res, E, G), = ctx.solve([p])
+    arr = (wlg.Problem * 1)(p)
+    a = [np.zeros(4 * N + 1, np.uint8), np.zeros(2 * N, np.int8), np.zeros(24, np.int32), np.zeros(24, np.int32),
+         np.zeros(24 * N, np.int8)]
+    ptr = [x.ctypes.data_as(C.c_void_p) for x in a]
+    wlg.call("wlg_prerun", ctx._h, C.cast(arr, C.c_void_p), 1, *ptr)
+    r2, E2, G2 = (wlg.Result * 1)(), np.zeros(4 * N + 1, np.int32), np.zeros(4 * N + 1)
+    wlg.call("wlg_mainrun", ctx._h, C.cast(arr, C.c_void_p), 1, *ptr, 600.0, C.cast(r2, C.c_void_p),
+             E2.ctypes.data_as(C.c_void_p), G2.ctypes.data_as(C.c_void_p), len(E2))
+    assert res.status == 0 and r2[0].status == 0 and r2[0].outer_iterations == res.outer_iterations
+    n = r2[0].n_energies
+    assert np.array_equal(E2[:n], E) and np.array_equal(G2[:n], G)
