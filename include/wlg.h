@@ -199,7 +199,7 @@ typedef struct {
 typedef struct wlg_context wlg_context;
 
 /* A context owns a CUDA stream and the device buffers of the engine on
- * `device`, four auxiliary streams on which a batch's launch groups (by
+ * `device`, twelve auxiliary streams on which a batch's launch groups (by
  * kernel form and team size) run side by side, joined back to the solve's
  * stream by events, and host worker threads for the per-problem host phases
  * (started on first use).  mem_budget_bytes = 0 means no limit beyond the

@@ -203,13 +203,16 @@ inline int team_bytes(const MainDesc& d, int variant, int team)
 
 // The lattice storage of d: registers up to 64 sites, else bonds where a row's
 // right and down bonds fit one word (Y <= 16: two words read per proposal
-// instead of three rows and three couplings), else rows, else linear words.
+// instead of three rows and three couplings; periodic lattices, with no bond
+// missing, do without masks per row: 16x16 on every SM 0.322 -> 0.303 us a step),
+// else rows, else linear words.
 // Tight states keep rows, whose tables take no room.
 inline int lattice_store(const MainDesc& d, bool tight)
 {
   if (d.N <= 64) return d.X >= 3 && d.Y >= 3 ? kStoreTable : kStoreReg;
   if (d.rows == 0) return kStoreLinear;
-  return d.Y <= 16 && !tight ? kStoreBonds : kStoreRows;
+  if (d.Y > 16 || tight) return kStoreRows;
+  return d.boundary == 0 ? kStoreBonds : kStoreBondsOpen;
 }
 
 inline int tight_variant(const MainDesc& d) { return lattice_store(d, true) | kVariantGlobal | kVariantTight; }
@@ -234,8 +237,9 @@ inline int kernel_variant(const MainDesc& d, int team, bool resumable)
 {
   const int store = lattice_store(d, false);
   if (store == kStoreRows && !resumable) {
-    if (team_bytes(d, kStoreBonds2, team) <= kSmemBytes) return kStoreBonds2;
-    if (team_bytes(d, kStoreBonds2 | kVariantGlobal, team) <= kSmemBytes) return kStoreBonds2 | kVariantGlobal;
+    const int two = d.boundary == 0 ? kStoreBonds2 : kStoreBonds2Open;
+    if (team_bytes(d, two, team) <= kSmemBytes) return two;
+    if (team_bytes(d, two | kVariantGlobal, team) <= kSmemBytes) return two | kVariantGlobal;
   }
   if (team_bytes(d, store, team) <= kSmemBytes) return store;
   if (team_bytes(d, store | kVariantGlobal, team) <= kSmemBytes) return store | kVariantGlobal;

@@ -182,7 +182,18 @@ WLG_HD inline StateLayout state_layout(int P, int I, int nwL, int L)
 // row per shared word (lattice_rows).  Bonds: for rows of up to 16 sites, the
 // unsatisfied right bonds (low half) and down bonds (high half) of a row in one
 // word instead of its spins; for rows of up to 32, in two words.
-enum Store { kStoreLinear = 0, kStoreReg = 1, kStoreTable = 2, kStoreRows = 3, kStoreBonds = 4, kStoreBonds2 = 5 };
+enum Store {
+  kStoreLinear = 0,
+  kStoreReg = 1,
+  kStoreTable = 2,
+  kStoreRows = 3,
+  kStoreBonds = 4,   // periodic: no bond missing
+  kStoreBonds2 = 5,
+  kStoreBondsOpen = 6,
+  kStoreBonds2Open = 7
+};
+WLG_HD constexpr bool store_bonds(int store) { return store >= kStoreBonds; }
+WLG_HD constexpr bool store_two_words(int store) { return store == kStoreBonds2 || store == kStoreBonds2Open; }
 
 // Draws a walker keeps ahead (a power of two), and the bytes of a warp's ring
 // of them: slot after slot of 32 lanes, the first slot repeated at the end.
@@ -230,7 +241,7 @@ WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, boo
   t.off_ring = o;
   o = align16(o + (tight ? 0 : team / 32 * kRingWarpBytes));
   t.off_lat = o;  // the lattice, or the exchange staging of a register lattice
-  o = align16(o + 4 * (reg ? 2 : (store == kStoreBonds2 ? 2 * d.nwL : d.nwL)) * team);
+  o = align16(o + 4 * (reg ? 2 : (store_two_words(store) ? 2 * d.nwL : d.nwL)) * team);
   t.off_E = o;
   o = align16(o + 4 * team);
   t.off_perm = o;
@@ -240,7 +251,7 @@ WLG_HD inline TeamLayout team_layout(const MainDesc& d, int team, int store, boo
   t.off_J = o;
   o = align16(o + 4 * 2 * d.nwL);
   t.off_tab = o;  // neighbour table and degrees per site, or bond masks per column and per row
-  o = align16(o + (store == kStoreTable ? 20 * d.N : (store >= kStoreBonds ? align16(8 * d.Y) + 16 * d.X : 0)));
+  o = align16(o + (store == kStoreTable ? 20 * d.N : (store_bonds(store) ? align16(8 * d.Y) + 16 * d.X : 0)));
   t.off_f = o;  // f [I], then ln f [I]
   o = align16(o + 16 * I);
   t.off_cond = o;

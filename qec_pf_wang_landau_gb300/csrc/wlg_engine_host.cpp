@@ -248,7 +248,7 @@ struct wlg_context {
   size_t used = 0;
   DevBuf buf[kSlots];
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  static constexpr int kAux = 4;
+  static constexpr int kAux = 12;  // launch groups of a mixed batch: storages, boundaries and team sizes
   cudaStream_t aux[kAux] = {};          // main-run groups side by side
   cudaEvent_t aux_ev[kAux + 1] = {};    // fork, then one join per aux stream
   void release_aux()

@@ -137,8 +137,8 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
 {
   constexpr bool kTable = kStore == kStoreTable;
   constexpr bool kReg = kStore == kStoreReg || kTable;
-  constexpr bool kTwo = kStore == kStoreBonds2;
-  constexpr bool kBonds = kStore == kStoreBonds || kTwo;
+  constexpr bool kTwo = store_two_words(kStore);
+  constexpr bool kBonds = store_bonds(kStore);
   const MainDesc& d = head.d;
   const int P = team.size;
   // start time straight into the result slot: a value kept live through the
@@ -747,6 +747,8 @@ MainFn main_fn_of(int store, bool tight)
     case kStoreRows: return WLG_MAIN_FN(kStoreRows);
     case kStoreBonds: return &k_main_batch<kStoreBonds, false, false, kMaxThreads>;
     case kStoreBonds2: return &k_main_batch<kStoreBonds2, false, false, kMaxThreads>;
+    case kStoreBondsOpen: return &k_main_batch<kStoreBondsOpen, false, false, kMaxThreads>;
+    case kStoreBonds2Open: return &k_main_batch<kStoreBonds2Open, false, false, kMaxThreads>;
     default: return WLG_MAIN_FN(kStoreLinear);
   }
 #undef WLG_MAIN_FN
@@ -762,6 +764,8 @@ MainFn main_fn_cluster_of(int store)
     case kStoreRows: return &k_main_batch<kStoreRows, false, true, kMaxThreads>;
     case kStoreBonds: return &k_main_batch<kStoreBonds, false, true, kMaxThreads>;
     case kStoreBonds2: return &k_main_batch<kStoreBonds2, false, true, kMaxThreads>;
+    case kStoreBondsOpen: return &k_main_batch<kStoreBondsOpen, false, true, kMaxThreads>;
+    case kStoreBonds2Open: return &k_main_batch<kStoreBonds2Open, false, true, kMaxThreads>;
     default: return &k_main_batch<kStoreLinear, false, true, kMaxThreads>;
   }
 }

@@ -427,7 +427,7 @@ WLG_HD inline SweepLayout sweep_layout(int X, int Y, int L, int lg)
 template <int kStore>
 __global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
 {
-  constexpr bool kBonds = kStore == kStoreBonds;
+  constexpr bool kBonds = store_bonds(kStore);
   extern __shared__ __align__(16) unsigned char smem[];
   const int groups = (a.wpi + 31) / 32, lane = threadIdx.x;
   const int k = blockIdx.x / groups, w = (blockIdx.x - k * groups) * 32 + lane, t = k * a.wpi + w;
@@ -853,7 +853,8 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
     return launch_status();
   }
   const int smem = sweep_layout(X, Y, a.L, lg).bytes;
-  const auto kernel = Y <= 16 ? &k_wl_sweep<kStoreBonds> : &k_wl_sweep<kStoreRows>;
+  const auto kernel =
+    Y > 16 ? &k_wl_sweep<kStoreRows> : (boundary == 0 ? &k_wl_sweep<kStoreBonds> : &k_wl_sweep<kStoreBondsOpen>);
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return WLG_ERR_CUDA;

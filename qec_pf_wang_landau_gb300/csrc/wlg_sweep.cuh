@@ -399,8 +399,10 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
   constexpr bool kTable = kStore == kStoreTable;
   constexpr bool kReg = kStore == kStoreReg || kTable;
   constexpr bool kRows = kStore == kStoreRows;
-  constexpr bool kTwo = kStore == kStoreBonds2;
-  constexpr bool kBonds = kStore == kStoreBonds || kTwo;
+  constexpr bool kTwo = store_two_words(kStore);
+  constexpr bool kBonds = store_bonds(kStore);
+  // bonds of periodic lattices: every row and column alike, no masks for rows
+  constexpr bool kMissing = kStore == kStoreBondsOpen || kStore == kStoreBonds2Open;
   // Pairs of steps unrolled in the persistent run, so that ptxas schedules
   // across them: 16x16 on every SM 0.368 -> 0.339 us a step, 12x12 0.157 ->
   // 0.148, 6x6 0.129 -> 0.122.  Not for the longer steps of rows and linear
@@ -569,12 +571,23 @@ __device__ __forceinline__ void wl_sweep(const SweepTeam& team, Walker<kTight>& 
       } else {
         const uint64_t xi = static_cast<uint64_t>(x) * uX;
         f.i = static_cast<uint32_t>(xi >> 32);
-        const uint64_t xj = static_cast<uint64_t>(static_cast<uint32_t>(xi)) * uY;
-        f.j = static_cast<uint32_t>(xj >> 32);
-        lo_s = static_cast<uint32_t>(xj);
+        const uint32_t rest = static_cast<uint32_t>(xi);
+        if constexpr (kBonds && !kMissing) {  // two products: 16x16 on every SM 3 % faster
+          f.j = __umulhi(rest, uY);
+          lo_s = rest * uY;
+        } else {
+          const uint64_t xj = static_cast<uint64_t>(rest) * uY;
+          f.j = static_cast<uint32_t>(xj >> 32);
+          lo_s = static_cast<uint32_t>(xj);
+        }
         if constexpr (kBonds) {
-          f.col = lds_u64(jt_a + 8 * f.j);
-          f.row = lds_u128(rt_a + 16 * f.i);
+          if constexpr (kMissing) {
+            f.col = lds_u64(jt_a + 8 * f.j);
+            f.row = lds_u128(rt_a + 16 * f.i);
+          } else {
+            f.col = make_uint2(lds_u32(jt_a + 8 * f.j), 0u);
+            f.row = make_uint4(0xFFFFFFFFu, kTwo ? 0xFFFFFFFFu : 0xFFFF0000u, 0u, 0u);
+          }
         }
       }
       f.ok = lo_s + d_thr >= 2u * d_thr;
