@@ -65,16 +65,17 @@ __device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* sme
 {
   constexpr int kW = kTwo ? 2 : 1;
   const int N = d.N, X = d.X, Y = d.Y, L = 4 * N + 1, tid = threadIdx.x;
-  const int threads = (d.walkers + 31) / 32 * 32, Lh = pre_hist_words(L);
+  const int lg = energy_step_log2(d.boundary), len = (4 * N >> lg) + 1;
+  const int threads = (d.walkers + 31) / 32 * 32, Lh = pre_hist_words(len);
   if (tid >= threads) return;  // warps beyond this problem's walkers
-  const PreLayout l = pre_layout(X, Y, L, d.n_int, threads);
+  const PreLayout l = pre_layout(X, Y, len, d.n_int, threads);
   uint32_t* hist = reinterpret_cast<uint32_t*>(smem + l.off_hist);
   uint32_t* thr = reinterpret_cast<uint32_t*>(smem + l.off_thr);
   uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
   uint32_t* base = reinterpret_cast<uint32_t*>(smem + l.off_base);
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
   uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
-  PreWalk p{X, Y, d.boundary, -2 * N, 2 * N, d.n_int, d.len_int, d.n_iter, threads, hist,
+  PreWalk p{X, Y, d.boundary, -2 * N, lg, len, 0, d.n_int, d.len_int, d.n_iter, threads, hist,
             reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr,
             col, row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words), found_pool + d.off_found};
   const PreSync sync{threads};
@@ -113,11 +114,14 @@ __device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* sme
   // wl.cu:261-340: minus the sum over bonds of s s J
   const int bonds = d.boundary == 0 ? 2 * N : 2 * N - X - Y;
   int E = 2 * static_cast<int>(unsat) - bonds;
+  p.bin0 = (E + 2 * N) & ((1 << lg) - 1);  // the lattice's energies start there
+  p.e_min += p.bin0;
   uint32_t s0 = base[0] & 1u;
   uint64_t pos = 0;
   pre_walk<kTwo, false, kKeys>(p, sync, w, w < d.walkers, key_u32(d.seed, static_cast<uint64_t>(d.sample)),
                         2 + static_cast<uint64_t>(w), pos, E, s0);
-  for (int q = tid; q < L; q += threads) seen_pool[d.off_seen + q] = hist[q] != 0 ? 1 : 0;
+  for (int q = tid; q < L; q += threads)
+    seen_pool[d.off_seen + q] = ((q - p.bin0) & ((1 << lg) - 1)) == 0 && hist[(q - p.bin0) >> lg] != 0 ? 1 : 0;
   for (int q = tid; q < d.n_int; q += threads) {
     const bool found = p.claim[q] != kPreEmpty;
     fflag_pool[d.off_fflag + q] = found ? 1 : 0;

@@ -42,6 +42,9 @@ struct PreDesc {
 // rounds.
 constexpr int kAcceptEntries = 27;
 WLG_HD inline int pre_hist_words(int len) { return (len + 4) & ~3; }  // one copy, a spare entry included
+// log2 of the distance between a lattice's energies: every site has four bonds
+// (periodic), or some fewer
+WLG_HD inline int energy_step_log2(int boundary) { return boundary == 0 ? 2 : 1; }
 WLG_HD inline bool pre_walk_fits(int X, int Y, int walkers, long long n_iter)
 {
   return X >= 2 && Y >= 2 && Y <= 32 && walkers <= 1024 && n_iter * walkers < (1ll << 31) &&
@@ -52,6 +55,7 @@ WLG_HD inline bool pre_walk_fits(int X, int Y, int walkers, long long n_iter)
 struct PreLayout {
   int off_hist, off_claim, off_foundE, off_thr, off_col, off_row, off_J, off_base, off_words, bytes;
 };
+// len_hist: energies of the range that a walker can have
 WLG_HD inline PreLayout pre_layout(int X, int Y, int len_hist, int n_int, int threads)
 {
   auto up = [](long long x) { return static_cast<int>((x + 15) & ~15ll); };

@@ -104,7 +104,8 @@ __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char*
 {
   constexpr int kW = kTwo ? 2 : 1;
   const int k = blockIdx.x, w = threadIdx.x, X = a.X, Y = a.Y, N = X * Y;
-  const int threads = blockDim.x, len = a.E_max - a.E_min + 1, Lh = pre_hist_words(len);
+  const int lg = energy_step_log2(a.boundary), all = a.E_max - a.E_min + 1, len = ((all - 1) >> lg) + 1;
+  const int threads = blockDim.x, Lh = pre_hist_words(len);
   const bool live = w < a.wpi;
   const size_t t = static_cast<size_t>(k) * a.wpi + w;
   const PreLayout l = pre_layout(X, Y, len, a.n_int, threads);
@@ -113,13 +114,18 @@ __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char*
   uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
   uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
-  const PreWalk p{X, Y, a.boundary, a.E_min, a.E_max, a.n_int, min(a.len_int, 1 << 15), a.n_iter, threads, hist,
+  PreWalk p{X, Y, a.boundary, a.E_min, lg, len, 0, a.n_int, min(a.len_int, 1 << 15), a.n_iter, threads, hist,
                   reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr, col,
                   row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words),
                   a.found_lat + static_cast<long long>(k) * a.n_int * N};
   const PreSync sync{threads};
+  // all walkers of a sample have energies a step apart (k_prerun)
+  p.bin0 = (a.E[static_cast<size_t>(k) * a.wpi] - a.E_min) & ((1 << lg) - 1);
+  p.e_min += p.bin0;
+  p.len = (all - 1 - p.bin0 >> lg) + 1;
   for (int q = w; q < Lh; q += threads) {
-    const uint32_t h = q < len ? static_cast<uint32_t>(a.H[static_cast<size_t>(k) * len + q]) : 0u;
+    const int e = p.bin0 + (q << lg);
+    const uint32_t h = e < all ? static_cast<uint32_t>(a.H[static_cast<size_t>(k) * all + e]) : 0u;
     hist[q] = hist[Lh + q] = h;
   }
   for (int q = w; q < a.n_int; q += threads)
@@ -165,7 +171,7 @@ __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char*
   }
   pre_walk<kTwo, true, kKeys>(p, sync, w, live, key_u32(a.seed, static_cast<uint64_t>(k)), 2 + static_cast<uint64_t>(w), pos, E,
                        s0);
-  for (int q = w; q < len; q += threads) a.H[static_cast<size_t>(k) * len + q] = hist[q];
+  for (int q = w; q < p.len; q += threads) a.H[static_cast<size_t>(k) * all + p.bin0 + (q << lg)] = hist[q];
   for (int q = w; q < a.n_int; q += threads)
     if (p.claim[q] != kPreEmpty && p.claim[q] != 0u) a.flag_found[static_cast<size_t>(k) * a.n_int + q] = 1;
   if (live) {
@@ -293,6 +299,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
       const int8_t* s = a.lat + a.off_lat[t];
       for (int q = 0; q < N; ++q) fast = fast && (s[q] == 1 || s[q] == -1);
       fast = fast && (a.seed_off[t] & 1u) == 0;
+      // energies on one grid, as the lattices of one sample have them
+      fast = fast && ((a.E[t] - a.E[static_cast<size_t>(k) * a.wpi]) & ((1 << energy_step_log2(a.boundary)) - 1)) == 0;
     }
   }
   if (__syncthreads_and(fast ? 1 : 0) == 0) {
@@ -803,7 +811,8 @@ wlg_status wlg_wang_landau_pre_run(int* d_energy, int* d_flag_found_interval, in
                d_offset_lattice, E_min, E_max, num_iterations, X, Y, seed, static_cast<int>(num_intervals), len_interval,
                walker_per_sample, boundary, 0};
   if (static_cast<long long>(X) * Y <= 4096 && pre_walk_fits(X, Y, walker_per_sample, num_iterations)) {
-    const size_t bytes = static_cast<size_t>(pre_layout(X, Y, len_hist, a.n_int, threads).bytes);
+    const size_t bytes = static_cast<size_t>(
+      pre_layout(X, Y, ((len_hist - 1) >> energy_step_log2(boundary)) + 1, a.n_int, threads).bytes);
     if (bytes <= 227 * 1024) {
       a.bonds = 1;
       smem = std::max(smem, bytes);

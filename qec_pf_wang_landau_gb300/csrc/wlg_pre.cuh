@@ -11,6 +11,8 @@
 //   * a claim on a coarse bin is the key (round + 1) << 10 | walker under
 //     atomicMin, so no later round undercuts it; the winner's lattice is
 //     stored after the next barrier;
+//   * the histogram has an entry per energy the lattice can have (every 2nd or
+//     4th), or its loads and atomics would share 8 of the 32 banks;
 //   * lattices are kept as unsatisfied bonds, a row of right bonds and of down
 //     bonds in one word (up to 16 columns) or two (up to 32), [word][walker],
 //     plus the spin of site 0: a proposal reads two or three words and no
@@ -24,11 +26,11 @@
 // them, and rare cases sit in one warp-uniform block so that nothing else
 // branches).  GB300, 128 walkers a sample, time per round, against int8 lattices
 // with 64-bit counts, an acceptance table read after the histogram and two
-// barriers: 24x24 1.09 -> 0.21 us, 16x16 1.12 -> 0.19 us; 120 uneven lattices of
-// 4-16 a side 27.3 -> 4.8 ms; the operator, 64 samples of 9x9, 1000 rounds, with
-// set-up 2.05 -> 0.31 ms.  On the way: branches around site fallback and claims
-// 0.40 us a round, a branch in the barrier, around the lattice stores and a load
-// of the claim each round 0.26 us.
+// barriers: 24x24 1.09 -> 0.18 us, 16x16 1.12 -> 0.16 us; 120 uneven lattices of
+// 4-16 a side 27.3 -> 4.4 ms; the operator, 64 samples of 9x9, 1000 rounds, with
+// set-up 2.05 -> 0.28 ms.  On the way: branches around site fallback and claims
+// 0.40 us a round; a branch in the barrier, around the lattice stores and a load
+// of the claim each round 0.26; a histogram entry per energy value 0.21.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -77,7 +79,7 @@ __device__ __forceinline__ void fill_accept(uint32_t* acc_thr, int tid)
 }
 
 // The largest t >= 0 with x < acc_thr[t], or -1.  -log u names it up to one.
-__device__ __forceinline__ int accept_limit(uint32_t x, const uint32_t* acc_thr)
+__device__ __noinline__ int accept_limit(uint32_t x, const uint32_t* acc_thr)
 {
   const int k = max(static_cast<int>(-log_uniform(x)), 0);
   return k - 1 + (x < acc_thr[k] ? 1 : 0) + (x < acc_thr[k + 1] ? 1 : 0);
@@ -100,10 +102,12 @@ __device__ __forceinline__ void store_if(bool p, uint32_t* a, uint32_t v)
 // A sample's walk: where its pieces lie and its parameters.
 struct PreWalk {
   int X, Y, boundary;
-  int e_min, e_max;  // histogram range
+  int e_min, lg;       // lowest energy a walker can have in the range; energies lie 2^lg apart
+  int len;             // such energies in the range
+  int bin0;            // e_min above the first coarse bin's edge
   int n_int, len_int, n_iter;
   int threads;         // walkers, rounded up to a warp
-  uint32_t* hist;      // [2][pre_hist_words(e_max - e_min + 1)], both copies the same
+  uint32_t* hist;      // [2][pre_hist_words(len)], both copies the same
   uint32_t* claim;     // [n_int]: kPreEmpty, the winner's key, or 0 (stored before the walk)
   int* found_E;        // [n_int] energy of the stored lattice
   const uint32_t* acc_thr;
@@ -154,7 +158,7 @@ __device__ __forceinline__ void bond_words(uint32_t r, uint32_t dn, uint32_t Jr,
 // row by row: along column 0 and then along the row, a bond flips the spin when
 // coupling bit and unsatisfied bit differ.  s0: site 0's spin bit.
 template <bool kTwo>
-__device__ __forceinline__ void store_spins(const PreWalk& p, int w, uint32_t s0, int8_t* dst)
+__device__ __noinline__ void store_spins(const PreWalk& p, int w, uint32_t s0, int8_t* dst)
 {
   constexpr int kW = kTwo ? 2 : 1;
   for (int i = static_cast<int>(threadIdx.x & 31u); i < p.X; i += 32) {
@@ -177,7 +181,7 @@ struct Copy {
 };
 
 // The walk of this thread's walker `w` (live: it exists).  E, s0 and pos (draws
-// consumed, even) are updated; kRange: a proposal outside [e_min, e_max]
+// consumed, even) are updated; kRange: a proposal outside the range
 // stops the walker (wl.cu:522-529) and leaves its energy in E.  Every thread of
 // the CTA's first p.threads calls it.  On return both copies of the histogram
 // hold all visits.
@@ -187,7 +191,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
 {
   constexpr int kW = kTwo ? 2 : 1;
   const int T = p.threads, X = p.X, Y = p.Y, N = X * Y;
-  const int Lh = pre_hist_words(p.e_max - p.e_min + 1);
+  const int Lh = pre_hist_words(p.len), lg = p.lg;
   const int spare = Lh - 1;  // takes the visits of threads without a walker
   const uint32_t site_thr = static_cast<uint32_t>(N) * 2048u + 16384u;
   const double site_scale = (N - 1 + 0.999999);
@@ -198,8 +202,8 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   const uint32_t s_lo = static_cast<uint32_t>(subseq), s_hi = static_cast<uint32_t>(subseq >> 32);
   uint32_t* lat = p.words + w;
   bool ok = live;
-  if (kRange) ok = ok && E >= p.e_min && E <= p.e_max;
-  int io = ok ? E - p.e_min : spare;
+  if (kRange) ok = ok && E >= p.e_min && (E - p.e_min) >> lg < p.len;
+  int io = ok ? (E - p.e_min) >> lg : spare;
   int hit_before = spare;
   int e_start = io;     // batched walk: the one bin visited without a move into it
   int want = -1;        // coarse bin claimed in the round before
@@ -237,7 +241,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
       na ^= ma;
       nb ^= mb;
     }
-    in = io + 2 * (4 - static_cast<int>(c.y + m.z) - 2 * static_cast<int>(unsat));
+    in = io + (2 * (4 - static_cast<int>(c.y + m.z) - 2 * static_cast<int>(unsat)) >> lg);
   };
   // Prepares the next round from its two draws, and claims the coarse bin of
   // this round's move when it is still empty (`key`: this round's).  What is
@@ -257,12 +261,13 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
     limit = __float_as_int(big) - 0x4B400000 - (away < 0.0f ? 1 : 0);
     const bool close = fabsf(away) < 2.0f * kLogAbsErr;
     auto coarse = [&]() {
-      return min(len_one ? io : static_cast<int>(__umulhi(static_cast<uint32_t>(io), len_magic)), p.n_int - 1);
+      const int n = p.bin0 + (io << lg);
+      return min(len_one ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), len_magic)), p.n_int - 1);
     };
     bool empty = kRange ? moved & (p.claim[coarse()] >= key_now) : moved & (fresh | (io == e_start));
     claims = false;
     want = -1;
-    if (__any_sync(0xFFFFFFFFu, edge | close | empty)) {
+    if (__any_sync(0xFFFFFFFFu, edge | close | empty)) [[unlikely]] {
       if (edge) {
         const uint32_t site = static_cast<uint32_t>(site_exact(x_site, site_scale)), i = site / static_cast<uint32_t>(Y);
         propose(i, site - i * static_cast<uint32_t>(Y));
@@ -292,7 +297,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
       const int bin = __shfl_sync(0xFFFFFFFFu, want, lane);
       const int e = __shfl_sync(0xFFFFFFFFu, io, lane);
       const uint32_t s = __shfl_sync(0xFFFFFFFFu, s0, lane);
-      if (static_cast<int>(threadIdx.x & 31u) == lane) p.found_E[bin] = e + p.e_min;
+      if (static_cast<int>(threadIdx.x & 31u) == lane) p.found_E[bin] = (e << lg) + p.e_min;
       store_spins<kTwo>(p, (w & ~31) + lane, s, p.found_lat + static_cast<long long>(bin) * N);
       __syncwarp();
     }
@@ -302,14 +307,14 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   auto round = [&](auto copy, uint32_t x_site, uint32_t x_acc, auto beside) {
     constexpr int kCopy = decltype(copy)::value;
     sync();
-    if (claims) settle();
+    if (claims) [[unlikely]] settle();
     const uint32_t* now = p.hist + kCopy * Lh;
     uint32_t* other = p.hist + (1 - kCopy) * Lh;
     bool can = ok;
     if (kRange) {
-      if (ok && (in < 0 || in > p.e_max - p.e_min)) {  // the walker stops and keeps the offending energy
+      if (ok && (in < 0 || in >= p.len)) {  // the walker stops and keeps the offending energy
         ok = can = false;
-        E = in + p.e_min;
+        E = in * (1 << lg) + p.e_min;
         pos += 1;  // it consumed the site's draw alone
       }
     }
@@ -361,7 +366,9 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   uint4 a = four();
   prepare(a.x, a.y, false, false, claim_key);
   int left = p.n_iter;
-#pragma unroll 2
+  // not unrolled, rare cases out of line: the loop then stays in the instruction
+  // cache (16x16 0.181 -> 0.161 us a round)
+#pragma unroll 1
   for (; left >= 2; left -= 2) {
     uint4 b;
     round(Copy<0>{}, a.z, a.w, [&] { b = four(); });
@@ -370,7 +377,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
   }
   if (left > 0) round(Copy<0>{}, a.z, a.w, [] {});
   if (!kRange) pos = pos_in + 2 * static_cast<uint64_t>(p.n_iter);
-  if (ok) E = io + p.e_min;
+  if (ok) E = (io << lg) + p.e_min;
   // the last round's claims and visits
   sync();
   if (claims) settle();
