@@ -398,7 +398,9 @@ __global__ void k_wang_landau(const SweepArgs a)
   sweep_global(a, t);
 }
 
-// Shared memory of k_wl_sweep: one warp of 32 walkers (bytes).
+// Shared memory of k_wl_sweep: 32 walkers (bytes).
+constexpr int kSweepWarps = 8;  // at most
+static_assert(8 * 32 * kSweepWarps <= kRingWarpBytes);
 struct SweepLayout {
   int off_desc, off_J, off_tab, off_ring, off_lat, off_pair, bytes;
 };
@@ -422,33 +424,84 @@ WLG_HD inline SweepLayout sweep_layout(int X, int Y, int L, int lg)
   return l;
 }
 
+// Warps a block: helpers while all blocks fit beside each other (152 SMs, two
+// blocks of 8 warps each or four of 4 by their registers), one warp beyond,
+// each lane packing its own walker.  1 / 4 / 8 warps, us for 1 and 1000 steps:
+// 10x10, 32 blocks 27 199 / 21 180 / 17 173; 10x10, 512 blocks 40 212 / 25 187 /
+// 33 343 (two waves); 6x6, 1024 blocks 21 211 / 31 324 / 47 619.
+inline int sweep_warps(int blocks)
+{
+  return blocks <= 2 * 152 ? kSweepWarps : (blocks <= 4 * 152 ? kSweepWarps / 2 : 1);
+}
+
 // The sweep of the persistent main run (wlg_sweep.cuh) on the caller's arrays:
-// one warp takes 32 walkers of a sample, packs their lattices (bonds or rows)
-// and the bins of their windows into shared memory, and writes lattices,
-// visits and log g back at the end.  The step on global memory is one chain of
-// dependent loads and an FP64 exp, about 2.6 us; here 0.13 us, and packing and
-// unpacking cost some 10 us a call.  GB300: an outer iteration of 16 samples of
-// 10x10 on the operators (1024 walkers, 200 steps) 0.56 -> 0.047 ms, a whole run
-// of 16 samples of 6x6 on them 45 -> 5.5 ms.  Warps with arrays the sweep does
-// not take (couplings or spins other than +-1, log g of 2^100 and more, factors below 1, an energy
-// outside its window, windows wider than the columns) walk on global memory.
+// the first warp of a block walks 32 walkers of a sample.  All its warps pack
+// the lattices (bonds or rows) and the bins of the windows into shared memory,
+// and write lattices, visits and log g back at the end: a warp reads and writes
+// a lattice 32 sites at a time, and the bins of the walkers are dealt out over
+// the warps, because these short chains of dependent global loads, not bytes,
+// are what a short sweep spends its time on.
+// The step on global memory is one chain of dependent loads and an FP64 exp,
+// about 2.6 us; here 0.13 us.  With helpers, loads that do not wait for each
+// other and the shadows made while packing, a call of one step took, us: 1024
+// walkers of 10x10 34 -> 17, 8192 of 6x6 23 -> 15; of 200 steps 84 -> 52 and
+// 61 -> 50; 81 920 walkers, 1000 steps: 10x10 599 -> 562, 6x6 411 -> 440.  A run
+// of 16 samples of 6x6 on the operators 5.4 -> 5.0 ms (45 with the step on
+// global memory).
+// Warps with arrays the sweep does not take (couplings or spins other than
+// +-1, log g of 2^100 and more, factors below 1, an energy outside its window,
+// windows wider than the columns) walk on global memory.
 template <int kStore>
-__global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
+__global__ void __launch_bounds__(32 * kSweepWarps) k_wl_sweep(const SweepArgs a)
 {
   constexpr bool kBonds = store_bonds(kStore);
+  constexpr unsigned kAll = 0xFFFFFFFFu;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int groups = (a.wpi + 31) / 32, lane = threadIdx.x;
+  const int groups = (a.wpi + 31) / 32, tid = threadIdx.x, nt = blockDim.x;
+  const int lane = tid & 31, warp = tid >> 5, warps = nt >> 5;
+  // every warp: a lane per walker
   const int k = blockIdx.x / groups, w = (blockIdx.x - k * groups) * 32 + lane, t = k * a.wpi + w;
   const bool live = w < a.wpi && t < a.num_lattices;
   if (a.cond_inter[k] == -1) return;
+  const unsigned wmask = __ballot_sync(kAll, live);
   const int X = a.X, Y = a.Y, N = X * Y, lg = a.boundary == 0 ? 2 : 1, guard = guard_bins(lg);
   const bool open = a.boundary != 0;
+  const uint32_t row_mask = Y == 32 ? kAll : (1u << Y) - 1u;
   const SweepLayout l = sweep_layout(X, Y, a.L, lg);
   MainDesc& d = *reinterpret_cast<MainDesc*>(smem + l.off_desc);
   uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
-  uint32_t* words = reinterpret_cast<uint32_t*>(smem + l.off_lat) + lane;
+  uint32_t* words = reinterpret_cast<uint32_t*>(smem + l.off_lat);  // word r of walker q: [r * 32 + q]
+  float2* top = reinterpret_cast<float2*>(smem + l.off_ring);  // until the walk begins
   float2* pair = reinterpret_cast<float2*>(smem + l.off_pair) + guard * 32 + lane;
-  if (lane == 0) {
+  const long long at = live ? a.off_lat[t] : 0;
+  bool ok = true;
+  // sites to words of 32
+  const int nw = (N + 31) / 32;
+  if (warps == 1) {  // a lane a walker
+    for (int c = 0; c < nw && live; ++c) {
+      const int8_t* s = a.lat + at + c * 32;
+      const int n = min(32, N - c * 32);
+      uint32_t bits = 0;
+#pragma unroll 8
+      for (int j = 0; j < n; ++j) {
+        const int v = s[j];
+        ok = ok && (v == 1 || v == -1);
+        bits |= v < 0 ? 1u << j : 0u;
+      }
+      words[c * 32 + lane] = bits;
+    }
+  } else {
+#pragma unroll 8
+    for (int x = warp; x < 32 * nw; x += warps) {
+      const int q = x & 31, site = (x >> 5) * 32 + lane;
+      const int8_t* s = a.lat + __shfl_sync(kAll, at, q);
+      const int v = ((wmask >> q) & 1u) != 0 && site < N ? s[site] : 1;
+      ok = ok && (v == 1 || v == -1);
+      const uint32_t bits = __ballot_sync(kAll, v < 0);
+      if (lane == 0) words[x] = bits;
+    }
+  }
+  if (tid == 0) {
     d.X = X;
     d.Y = Y;
     d.N = N;
@@ -458,118 +511,169 @@ __global__ void __launch_bounds__(32) k_wl_sweep(const SweepArgs a)
     d.site_scale = (N - 1 + 0.999999);
     d.site_magic = a.magic;
   }
-  bool ok = true;
   const int8_t* Jk = a.J + static_cast<size_t>(k) * 2 * N;
-  for (int q = lane; q < 2 * X; q += 32) {  // coupling bits: right, then down
+  for (int q = nt - 1 - tid; q < 2 * X; q += nt) {  // coupling bits: right, then down
     const int8_t* src = Jk + q * Y;
     uint32_t bits = 0;
+#pragma unroll 8
     for (int j = 0; j < Y; ++j) {
-      ok = ok && (src[j] == 1 || src[j] == -1);
-      bits |= src[j] < 0 ? 1u << j : 0u;
+      const int v = src[j];
+      ok = ok && (v == 1 || v == -1);
+      bits |= v < 0 ? 1u << j : 0u;
     }
     Jr[q] = bits;
   }
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_tab);
-  fill_bond_tables<false>(col, reinterpret_cast<uint4*>(smem + l.off_tab + align16(8 * Y)), X, Y, open, 2 * (256 >> lg), lane, 32);
-  __syncwarp();
+  fill_bond_tables<false>(col, reinterpret_cast<uint4*>(smem + l.off_tab + align16(8 * Y)), X, Y, open, 2 * (256 >> lg),
+                          tid, nt);
   const int b = t / (a.wpi / a.n_int);
   const int e_first = a.start[k * a.n_int], e_last = a.end[k * a.n_int + a.n_int - 1];
   const int8_t* mask = a.spectrum + a.off_spec[k] - e_first;
   auto is_bad = [&](int En) { return En < e_first || En > e_last || mask[En] != 1; };
   Walker<false> wk;
-  wk.s0 = 0;
   wk.lo = wk.hi = wk.bb = wk.len = wk.E = 0;
-  int8_t* s = nullptr;
   double lnf = 0.0;
   unsigned long long* H = nullptr;
   double* G = nullptr;
+  bool frozen = true;
+  Split gs{0.0f, 0.0f};
+  float amax = 0.0f;
+  int ghi = 0;
   if (live) {
-    s = a.lat + a.off_lat[t];
-    auto row_bits = [&](int i) {
-      uint32_t r = 0;
-      for (int j = 0; j < Y; ++j) {
-        const int8_t v = s[i * Y + j];
-        ok = ok && (v == 1 || v == -1);
-        r |= v < 0 ? 1u << j : 0u;
-      }
-      return r;
-    };
-    const uint32_t first = row_bits(0);
-    uint32_t r = first;
-    for (int i = 0; i < X; ++i) {
-      const uint32_t below = i + 1 < X ? row_bits(i + 1) : first;
-      words[i * 32] = kBonds ? bond_word(r, below, Jr[i], Jr[X + i], Y, open, i + 1 == X) : r;
-      r = below;
-    }
-    wk.s0 = first & 1u;
     wk.E = a.E[t];
     wk.lo = a.start[b];
     wk.hi = a.end[b];
-    ok = ok && wk.E >= wk.lo && wk.E <= wk.hi;
+    frozen = a.cond[b] != 0;
+    bool own = wk.E >= wk.lo && wk.E <= wk.hi;
     wk.bb = wk.lo + ((wk.E - wk.lo) & ((1 << lg) - 1));  // the walker's energies, a step apart
     wk.len = ((wk.hi - wk.bb) >> lg) + 1;
-    ok = ok && wk.len <= a.L;
+    own = own && wk.len <= a.L;
     lnf = log(a.factor[t]);
-    ok = ok && lnf >= 0.0 && lnf < 1e6;
+    own = own && lnf >= 0.0 && lnf < 1e6;
     H = a.H + a.off_hist[t] + (wk.bb - wk.lo);
     G = a.logG + a.off_hist[t] + (wk.bb - wk.lo);
-    if (ok)
-      for (int c = 0; c < wk.len; ++c) ok = ok && (__double2hiint(G[c << lg]) & 0x7FFFFFFF) < 0x46300000;  // |g| < 2^100
+    if (own) {  // bins with their shadows (wl_sweep)
+      const double gbase = G[wk.E - wk.bb];
+      gs = split_of<true>(gbase);
+      ghi = __double2hiint(gbase) & 0x7FFFFFFF;
+#pragma unroll 4
+      for (int c = warp - guard; c < wk.len + guard; c += warps) {
+        const int En = wk.bb + c * (1 << lg);
+        const bool bad = is_bad(En), in = En >= wk.lo && En <= wk.hi;
+        const double g = in ? G[c * (1 << lg)] : 0.0;
+        const int g_hi = __double2hiint(g) & 0x7FFFFFFF;
+        own = own && g_hi < 0x46300000;  // |g| < 2^100
+        const float shadow = shadow_of<true>(g, gs);
+        if (in && !bad) {
+          amax = fmaxf(amax, fabsf(shadow));
+          ghi = max(ghi, g_hi);
+        }
+        pair[c * 32] = make_float2(bad ? __int_as_float(0x7FC00000) : (in ? shadow : __int_as_float(0x7F800000)), 0.0f);
+      }
+    }
+    ok = ok && own;
   }
-  if (__any_sync(0xFFFFFFFFu, !ok)) {
-    if (live) sweep_global(a, t);
+  top[warp * 32 + lane] = make_float2(amax, __int_as_float(ghi));
+  if (__syncthreads_or(!ok)) {
+    if (live && warp == 0) sweep_global(a, t);
     return;
   }
-  const unsigned wmask = __ballot_sync(0xFFFFFFFFu, live);
-  if (!live) return;
-  for (int c = -guard; c < wk.len + guard; ++c) {
-    const int En = wk.bb + c * (1 << lg);
-    pair[c * 32] = make_float2(is_bad(En) ? __int_as_float(0x7FC00000)
-                                          : (En >= wk.lo && En <= wk.hi ? 0.0f : __int_as_float(0x7F800000)),
-                               0.0f);
+  if (warp == 0) {
+    if (live) {
+      // words of 32 sites to rows, from the last: row i lies in words up to i
+      uint32_t* mine = words + lane;
+      auto row_at = [&](int i) {
+        const int bit = i * Y, f = bit >> 5, e = (bit + Y - 1) >> 5;
+        return __funnelshift_r(mine[f * 32], mine[e * 32], bit & 31) & row_mask;
+      };
+      const uint32_t first = mine[0] & row_mask;
+      for (uint32_t i = X, below = first; i-- > 0;) {
+        const uint32_t r = row_at(i);
+        mine[i * 32] = kBonds ? bond_word(r, below, Jr[i], Jr[X + i], Y, open, i + 1 == X) : r;
+        below = r;
+      }
+      wk.s0 = first & 1u;
+      wk.lt.r = 0;
+      wk.lt.a = shared_addr(words + lane);
+      wk.lt.stride = 128u;
+      wk.pair = pair;
+      wk.ring_a = shared_addr(smem + l.off_ring) + 4 * lane;
+      wk.rng.init(key_u32(a.seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(w), a.off_iter[t]);
+      wk.start();
+      for (int v = 0; v < warps; ++v) {
+        amax = fmaxf(amax, top[v * 32 + lane].x);
+        ghi = max(ghi, __float_as_int(top[v * 32 + lane].y));
+      }
+      __syncwarp(wmask);
+      wk.gs = gs;
+      wk.amax = amax;
+      wk.ghi = ghi;
+      wk.fresh = true;
+      const uint32_t tab_a = shared_addr(col);
+      const SweepTeam team{d, 32, tab_a, tab_a + align16(8 * Y), Jr, Jr + X, 0, 0};
+      int flag = 0;
+      auto log_g = [&](int c) { return G[c << lg]; };
+      auto new_energy = [&](int En, int) {
+        flag = t + 1;
+        a.newE[t] = En;
+      };
+      auto fold = [&](float, int, bool last) {
+        if (last) return;  // by all warps, below
+        wk.fresh = false;
+        if (frozen) return;
+        for (int c = 0; c < wk.len; ++c) {
+          const uint32_t n = static_cast<uint32_t>(pair[c * 32].y);
+          if (n == 0) continue;
+          pair[c * 32].y = 0.0f;
+          H[c << lg] += n;
+          G[c << lg] = add_times<true>(G[c << lg], lnf, n);
+        }
+      };
+      wl_sweep<kStore, false, true>(team, wk, wmask, a.n_iter, frozen, lnf, 0, log_g, is_bad, new_energy, fold);
+      if constexpr (kBonds) {  // to rows: down column 0, then along each row
+        uint32_t edge = wk.s0;
+        for (int i = 0; i < X; ++i) {
+          const uint32_t word = mine[i * 32];
+          uint32_t r = (word ^ Jr[i]) << 1;
+          r ^= r << 1;
+          r ^= r << 2;
+          r ^= r << 4;
+          r ^= r << 8;
+          mine[i * 32] = r ^ (0u - edge);
+          edge ^= ((word >> 16) ^ Jr[X + i]) & 1u;
+        }
+      }
+      a.found[t] = flag;
+      a.E[t] = wk.E;
+      a.off_iter[t] = wk.rng.pos;
+    }
+    __syncwarp();
   }
-  wk.lt.r = 0;
-  wk.lt.a = shared_addr(words);
-  wk.lt.stride = 128u;
-  wk.pair = pair;
-  wk.ring_a = shared_addr(smem + l.off_ring) + 4 * lane;
-  wk.rng.init(key_u32(a.seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(w), a.off_iter[t]);
-  wk.start();
-  const uint32_t tab_a = shared_addr(col);
-  const SweepTeam team{d, 32, tab_a, tab_a + align16(8 * Y), Jr, Jr + X, 0, 0};
-  const bool frozen = a.cond[b] != 0;
-  int flag = 0;
-  auto log_g = [&](int c) { return G[c << lg]; };
-  auto new_energy = [&](int En, int) {
-    flag = t + 1;
-    a.newE[t] = En;
-  };
-  auto fold = [&](float, int, bool) {
-    wk.fresh = false;
-    if (frozen) return;
-    for (int c = 0; c < wk.len; ++c) {
+  __syncthreads();
+  if (!frozen)
+    for (int c = warp; c < wk.len; c += warps) {
       const uint32_t n = static_cast<uint32_t>(pair[c * 32].y);
       if (n == 0) continue;
-      pair[c * 32].y = 0.0f;
       H[c << lg] += n;
       G[c << lg] = add_times<true>(G[c << lg], lnf, n);
     }
-  };
-  wl_sweep<kStore, false, true>(team, wk, wmask, a.n_iter, frozen, lnf, 0, log_g, is_bad, new_energy, fold);
-  // lattices: rows as they are; bonds down column 0, then along each row
-  uint32_t edge = wk.s0;
-  for (int i = 0; i < X; ++i) {
-    const uint32_t word = words[i * 32], turn = word ^ Jr[i];
-    uint32_t sp = edge;
-    for (int j = 0; j < Y; ++j) {
-      s[i * Y + j] = (kBonds ? sp : (word >> j) & 1u) != 0 ? -1 : 1;
-      sp ^= (turn >> j) & 1u;
+  if (warps == 1) {
+    for (int i = 0; i < X && live; ++i) {
+      const uint32_t r = words[i * 32 + lane];
+      int8_t* s = a.lat + at + i * Y;
+#pragma unroll 4
+      for (int j = 0; j < Y; ++j) s[j] = (r >> j) & 1u ? -1 : 1;
     }
-    edge ^= ((word >> 16) ^ Jr[X + i]) & 1u;
+    return;
   }
-  a.found[t] = flag;
-  a.E[t] = wk.E;
-  a.off_iter[t] = wk.rng.pos;
+#pragma unroll 4
+  for (int x = warp; x < 32 * nw; x += warps) {
+    const int q = x & 31, site = (x >> 5) * 32 + lane;
+    int8_t* s = a.lat + __shfl_sync(kAll, at, q);
+    if (((wmask >> q) & 1u) == 0 || site >= N) continue;
+    const int i = static_cast<int>((static_cast<uint32_t>(site) * a.magic) >> 20);
+    s[site] = (words[i * 32 + q] >> (site - i * Y)) & 1u ? -1 : 1;
+  }
 }
 
 // -------------------------------------------------------------- flatness ----
@@ -868,7 +972,8 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return WLG_ERR_CUDA;
   const int samples = (num_lattices + walker_per_sample - 1) / walker_per_sample;
-  kernel<<<samples * ((walker_per_sample + 31) / 32), 32, smem, s>>>(a);
+  const int blocks = samples * ((walker_per_sample + 31) / 32);
+  kernel<<<blocks, 32 * sweep_warps(blocks), smem, s>>>(a);
   return launch_status();
 }
 

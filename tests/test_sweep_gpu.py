@@ -49,3 +49,18 @@ def test_sweep_operator_edges(cuda, X, Y, boundary, R, I, W, overlap, prob, n_it
         o_wang_landau(st, n_iter, seed)
         dev.wang_landau(n_iter, seed)
         assert_state_equal(dev.snapshot(), st, f"sweep {it}")
+
+
+# blocks of 8, 4 and 1 warps: up to 304, up to 608 and more blocks of 32 walkers
+HELPERS = [(4, 4, 0, 61, 2, 80), (4, 4, 1, 61, 2, 74), (4, 4, 0, 122, 2, 80), (3, 4, 1, 122, 2, 77), (40, 3, 0, 3, 6, 9)]
+
+
+@pytest.mark.parametrize("X,Y,boundary,R,I,W", HELPERS)
+def test_sweep_operator_helpers(cuda, X, Y, boundary, R, I, W):
+    seed = 777
+    st = mainrun_state(prerun_outputs(X, Y, boundary, 0.06, "i", seed, R, 64, min(16, X * Y), 60 * X * Y), I, W, 0.25)
+    dev = Dev(cuda, copy_state(st))
+    for it in range(3):
+        o_wang_landau(st, 40, seed)
+        dev.wang_landau(40, seed)
+        assert_state_equal(dev.snapshot(), st, f"sweep {it}")
