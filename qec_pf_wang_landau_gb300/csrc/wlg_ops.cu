@@ -677,7 +677,8 @@ __global__ void __launch_bounds__(32 * kSweepWarps) k_wl_sweep(const SweepArgs a
 }
 
 // -------------------------------------------------------------- flatness ----
-// wl.cu:892-967, one block per window, one thread per walker.
+// wl.cu:892-967, one block per window, a warp per walker: the loads of a
+// histogram do not wait for each other.
 __global__ void k_check_histogram(unsigned long long* __restrict__ H, double* __restrict__ factor,
                                   int8_t* __restrict__ cond, const int* __restrict__ off_hist,
                                   const int* __restrict__ end, const int* __restrict__ start,
@@ -685,36 +686,41 @@ __global__ void k_check_histogram(unsigned long long* __restrict__ H, double* __
                                   const int* __restrict__ cond_inter, double alpha, int W, int wpi, int n_int)
 {
   const int b = blockIdx.x;
-  const int w = threadIdx.x;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int k = (b * W) / wpi;
   if (cond[b] == 1 || cond_inter[k] == -1) return;
   const int len = end[b] - start[b] + 1;
   const int8_t* mask = spectrum + off_spec[k] + start[b] - start[k * n_int];
-  int flat = 0;
-  if (w < W) {
+  bool flat = true;
+  for (int w = threadIdx.x >> 5; w < W && flat; w += warps) {
     const unsigned long long* h = H + off_hist[b * W + w];
     unsigned long long mn = 2147483647ull;
     unsigned long long sum = 0;  // exact: the reference's double sum of integers is exact below 2^53
     int cnt = 0;
-    for (int i = 0; i < len; ++i) {
-      if (mask[i] != 1) continue;
+#pragma unroll 4
+    for (int i = lane; i < len; i += 32) {
       const unsigned long long v = h[i];
-      mn = v < mn ? v : mn;
-      sum += v;
-      ++cnt;
+      const bool on = mask[i] == 1;
+      mn = on && v < mn ? v : mn;
+      sum += on ? v : 0ull;
+      cnt += on ? 1 : 0;
     }
-    if (cnt > 0) {
-      const double avg = static_cast<double>(sum) / cnt;
-      flat = static_cast<double>(mn) >= alpha * avg ? 1 : 0;
+    for (int d = 16; d > 0; d >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, mn, d);
+      mn = o < mn ? o : mn;
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+      cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, d);
     }
+    const double avg = static_cast<double>(sum) / max(cnt, 1);
+    flat = cnt > 0 && static_cast<double>(mn) >= alpha * avg;
   }
-  const int n_flat = __syncthreads_count(flat);
-  if (n_flat == W && w < W) {
+  if (!__syncthreads_and(flat)) return;
+  for (int w = threadIdx.x >> 5; w < W; w += warps) {
     unsigned long long* h = H + off_hist[b * W + w];
-    for (int i = 0; i < len; ++i) h[i] = 0;
-    factor[b * W + w] = sqrt(factor[b * W + w]);
-    if (w == 0) cond[b] = 1;
+    for (int i = lane; i < len; i += 32) h[i] = 0;
   }
+  for (int w = threadIdx.x; w < W; w += blockDim.x) factor[b * W + w] = sqrt(factor[b * W + w]);
+  if (threadIdx.x == 0) cond[b] = 1;
 }
 
 // ------------------------------------------------------- log g averaging ----
@@ -774,24 +780,38 @@ __global__ void k_replica_exchange(int* __restrict__ off_lat, int* __restrict__ 
   if (cond_inter[k] == -1) return;
   const int w = threadIdx.x;
   const int t0 = b * W;
-  if (w == 0) {
-    Stream st;
-    st.init(key_i32(seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t0 % wpi), off_iter[t0]);
-    for (int i = W - 1; i > 0; --i) {
+  const int t = t0 + w;
+  // the permutation's draws by a thread each, its swaps by one in shared memory
+  __shared__ int swap[1024], order[1024];
+  Stream st;
+  uint64_t pos = 0;
+  int et = 0;
+  if (w < W) {
+    const uint64_t first = off_iter[t0];
+    if (w > 0) {
+      st.init(key_i32(seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t0 % wpi), first + (W - 1 - w));
       double u = st.uniform();
-      u *= (i + 0.999999);
-      const int r = static_cast<int>(trunc(u));
-      const int tmp = perm[t0 + i];
-      perm[t0 + i] = perm[t0 + r];
-      perm[t0 + r] = tmp;
+      u *= (w + 0.999999);
+      swap[w] = static_cast<int>(trunc(u));
     }
-    off_iter[t0] = st.pos;
+    order[w] = perm[t];
+    pos = w == 0 ? first + (W - 1) : off_iter[t];
+    et = E[t];
+  }
+  __syncthreads();
+  if (w == 0) {
+    for (int i = W - 1; i > 0; --i) {
+      const int r = swap[i], tmp = order[i];
+      order[i] = order[r];
+      order[r] = tmp;
+    }
   }
   __syncthreads();
   if (w >= W) return;
-  const int t = t0 + w;
-  const int o = W * (b + 1) + perm[t];
-  const int et = E[t], eo = E[o];
+  perm[t] = order[w];
+  if (w == 0) off_iter[t] = pos;
+  const int o = W * (b + 1) + order[w];
+  const int eo = E[o];
   if (et > end[b + 1] || et < start[b + 1]) return;
   if (eo > end[b] || eo < start[b]) return;
   const double gi_x = logG[off_hist[t] + et - start[b]];
@@ -799,8 +819,7 @@ __global__ void k_replica_exchange(int* __restrict__ off_lat, int* __restrict__ 
   const double gj_y = logG[off_hist[o] + eo - start[b + 1]];
   const double gj_x = logG[off_hist[o] + et - start[b + 1]];
   const double prob = fmin(1.0, exp(gi_x - gi_y) * exp(gj_y - gj_x));
-  Stream st;
-  st.init(key_i32(seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t % wpi), off_iter[t]);
+  st.init(key_i32(seed, static_cast<uint64_t>(k)), static_cast<uint64_t>(t % wpi), pos);
   if (st.uniform() < prob) {
     const int tmp = off_lat[t];
     off_lat[t] = off_lat[o];
@@ -988,7 +1007,7 @@ wlg_status wlg_check_histogram(unsigned long long* d_H, double* d_factor, int8_t
   if (W > 1024 || num_walker_total % W != 0) return WLG_ERR_INVALID;
   const int windows = num_walker_total / W;
   if (windows == 0) return WLG_OK;
-  k_check_histogram<<<windows, (W + 31) / 32 * 32, 0, as_stream(stream)>>>(
+  k_check_histogram<<<windows, std::min(W, 16) * 32, 0, as_stream(stream)>>>(
     d_H, d_factor, d_cond, d_offset_histogram, d_end, d_start, d_spectrum, d_offset_spectrum, d_cond_sample, alpha, W,
     walker_per_sample, num_intervals);
   return launch_status();

@@ -5,7 +5,8 @@ arrays that only the walk on global memory takes."""
 import numpy as np
 import pytest
 
-from tests.helpers import Dev, assert_state_equal, copy_state, mainrun_state, o_wang_landau, prerun_outputs
+from tests.helpers import (Dev, assert_state_equal, copy_state, mainrun_state, o_check_histogram, o_exchange,
+                           o_wang_landau, prerun_outputs)
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,23 @@ def test_sweep_operator_helpers(cuda, X, Y, boundary, R, I, W):
         o_wang_landau(st, 40, seed)
         dev.wang_landau(40, seed)
         assert_state_equal(dev.snapshot(), st, f"sweep {it}")
+
+
+@pytest.mark.parametrize("X,I,W", [(4, 3, 1), (6, 2, 16), (6, 4, 17), (4, 3, 33), (6, 1, 5), (4, 2, 1024)])
+def test_flatness_and_exchange_edges(cuda, X, I, W):
+    """One warp per walker up to 16, windows longer than a warp; permutations of 1 to 1024."""
+    st = mainrun_state(prerun_outputs(X, X, 0, 0.08, "i", 5, 2, 64, 16, 60 * X * X), I, W, 0.6)
+    rng = np.random.default_rng(I * W)
+    st["H"][:] = rng.integers(900, 1000, len(st["H"])).astype(np.uint64)
+    st["H"][len(st["H"]) // 2] = 100  # one window is not flat
+    st["logG"][:] = 3.0 * rng.random(len(st["logG"]))
+    dev = Dev(cuda, copy_state(st))
+    o_check_histogram(st, 0.8)
+    dev.check_histogram(0.8)
+    assert_state_equal(dev.snapshot(), st, "flatness")
+    assert st["cond"].any()
+    for it in range(3):
+        for even in (1, 0):
+            o_exchange(st, even, 5)
+            dev.exchange(even, 5)
+            assert_state_equal(dev.snapshot(), st, f"exchange {it}")
