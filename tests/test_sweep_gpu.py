@@ -85,3 +85,27 @@ def test_flatness_and_exchange_edges(cuda, X, I, W):
             o_exchange(st, even, 5)
             dev.exchange(even, 5)
             assert_state_equal(dev.snapshot(), st, f"exchange {it}")
+
+
+# a thread or a warp per lattice; Philox blocks that end inside a lattice
+@pytest.mark.parametrize("X,Y,nl,wpi", [(6, 8, 8192, 64), (6, 8, 8196, 4), (7, 7, 33, 3), (5, 9, 40, 8), (8, 16, 8200, 8),
+                                        (1, 3, 7, 7), (3, 1, 5, 5), (1, 128, 3, 1), (64, 2, 129, 3)])
+@pytest.mark.parametrize("boundary", [0, 1])
+def test_set_up_operators_edges(cuda, X, Y, nl, wpi, boundary):
+    import ctypes as C
+
+    import qec_pf_wang_landau_gb300 as wlg
+    import oracle as O
+    R, N = (nl + wpi - 1) // wpi, X * Y
+    p = lambda t: C.c_void_p(t.data_ptr())
+    J = cuda.zeros(R * 2 * N, dtype=cuda.int8, device="cuda")
+    lat = cuda.zeros(nl * N, dtype=cuda.int8, device="cuda")
+    E = cuda.zeros(nl, dtype=cuda.int32, device="cuda")
+    off = (np.arange(nl) * N).astype(np.int32)
+    wlg.call("wlg_init_interactions", p(J), N, R, 11, C.c_float(0.2), None)
+    wlg.call("wlg_init_lattice", p(lat), X, Y, nl, 11, wpi, None)
+    wlg.call("wlg_calc_energy", boundary, p(E), p(lat), p(J), p(cuda.from_numpy(off).cuda()), X, Y, nl, wpi, None)
+    h_J, h_lat = O.init_interactions(X, Y, R, 11, 0.2, "i"), O.init_lattice(X, Y, nl, 11, wpi)
+    assert np.array_equal(J.cpu().numpy(), h_J)
+    assert np.array_equal(lat.cpu().numpy(), h_lat)
+    assert np.array_equal(E.cpu().numpy(), O.calc_energy(boundary, h_lat, h_J, off, X, Y, nl, wpi))
