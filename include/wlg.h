@@ -281,11 +281,11 @@ wlg_status wlg_solve_raw(wlg_context* ctx, const wlg_problem* problems, int n, w
  * cudaMalloc: a framework that owns the device's whole memory pool, a
  * latency-critical loop that cannot take an allocation's implicit
  * synchronisation, a deployment that forbids allocating after start-up.
- * Every device buffer it needs comes from one fixed 8 MiB arena compiled
+ * Every device buffer it needs comes from one fixed 12 MiB arena compiled
  * into the library, which each GPU that loads the library holds until the
  * process exits.  A batch whose worst-case footprint (every window as wide
  * as the full energy range, including the global log g pool of problems too
- * large for shared memory) exceeds the arena is rejected with
+ * large for shared memory) exceeds 8 MiB of it is rejected with
  * WLG_ERR_CAPACITY before anything runs, leaving results and outputs as the
  * caller left them (400 problems of 6x6 lattices fit).  Runs on the current
  * device and `stream`; the call synchronises `stream` itself (after the

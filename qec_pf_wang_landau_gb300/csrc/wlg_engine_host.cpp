@@ -748,7 +748,7 @@ int spread_ranks(const Prepared& prep, int sms)
 
 constexpr int kTimedEpoch = 4;  // outer iterations per launch under a time limit
 
-// The main run of a prepared batch: one persistent launch per (form, team
+// The main run of a prepared batch: one persistent launch per (variant, team
 // size).  time_limit_s > 0: resumable launches of kTimedEpoch outer
 // iterations each, repeated until every problem finished or the limit
 // passed (the reference checks its time limit after each outer iteration,
@@ -777,7 +777,7 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   if (m == 0) return WLG_OK;
   int sms = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex.device);
-  // one launch per (form, team size); the form by lattice storage (fit_form)
+  // one launch per (variant, team size) (kernel_variant)
   std::map<std::pair<int, int>, std::vector<int>> groups;
   const bool resumable = time_limit_s > 0;
   const int spread = resumable ? 1 : spread_ranks(prep, sms);

@@ -22,7 +22,7 @@
 //   * spins: one u64 register for N <= 64 (with a neighbour table); for larger
 //     lattices with rows of up to 16 sites the unsatisfied bonds instead of the
 //     spins, so that a proposal reads two words and no couplings; one row per
-//     word up to 32 sites a row; else linear words.
+//     word (or its bonds in two) up to 32 sites a row; else linear words.
 //
 // Acceptance u < min(1, exp(dlogg)) is decided as log u < dlogg with FP32
 // values and a proven error bound.  What FP32 cannot settle (an acceptance
@@ -37,9 +37,9 @@
 // log g itself up to date (FP64 addition, shadow and count written back on every
 // change of energy, bins classified by a mask load, Philox in registers), time
 // per step of the longest problem, GB300: 6x6 0.29 -> 0.12 us (247 -> 97 warp
-// instructions), up to 12x12 mixed 0.35 -> 0.15 us, 16x16 with 512 walkers on
-// every SM 0.94 -> 0.36 us, 24x24 1.12 -> 0.63 us; between the sweeps, open
-// lattices of 7-11 with sweeps of 100 steps, 20.4 -> 15.1 ms per 400 iterations.
+// instructions), 12x12 0.35 -> 0.14 us, 16x16 with 512 walkers on every SM 0.94 ->
+// 0.30 us, 24x24 1.12 -> 0.62 us, four such problems over clusters 0.17 us; open
+// lattices of 7-11 with sweeps of 100 steps, 20.4 -> 10.9 ms per 400 iterations.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -5,7 +5,7 @@
 // it), latency-critical loops where an allocation's implicit
 // synchronisation is not acceptable, or hosts whose policy forbids
 // allocating after start-up.  For them the engine keeps one file-scope
-// arena of kNoAllocBytes (8 MiB) in device memory; every GPU that loads this
+// arena of kNoAllocBytes (12 MiB) in device memory; every GPU that loads this
 // library holds it until the process exits.  The no-allocation entry point
 // carves all of its device buffers out of this arena.
 //
