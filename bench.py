@@ -50,7 +50,7 @@ WORKLOAD = dict(X=6, Y=6, boundary=0, prob=0.04, seed=12345, samples=100, classe
 BYTES_PER_FLIP = 34  # log g read old + read new + write (24 B), histogram RMW (8 B), packed neighbourhood (~2 B)
 # DRAM bytes (read + write) of one main-run launch of this workload, from an ncu capture of the
 # bench's own launch (dram__bytes_read.sum + dram__bytes_write.sum); walker state never leaves the SM
-MAIN_TRAFFIC_BYTES = 797440
+MAIN_TRAFFIC_BYTES = 864256
 METRIC = "disorder samples converged/s (6x6 pbc p=0.04, 100 samples x 4 classes)"
 CPU_SAMPLE_PROBLEMS = 400  # the whole workload (samples 0-99 x ivhc)
 WORKLOAD_TAG = "6x6 pbc p.04 100x4cls pre128/32/1000 I10 W3 o.25 a.8 lnf1e-3 n1000 c20"
