@@ -227,8 +227,7 @@ struct Group {
   std::deque<Epoch> inflight;
   long long next_id = 0, completed = -1;
   std::vector<char> waited;  // per admission event: already waited on
-  int* d_order[kRing] = {};
-  int* d_next[kRing] = {};
+  int* d_order[kRing] = {};  // the queue's counter, then the problems in order: one copy an epoch
   int* h_order[kRing] = {};
   MainResult* h_snap[kRing] = {};
   cudaEvent_t ev[kRing] = {};
@@ -349,7 +348,6 @@ void wlg_server::teardown()
     if (g.stream != nullptr) cudaStreamSynchronize(g.stream);
     for (int b = 0; b < kRing; ++b) {
       cudaFree(g.d_order[b]);
-      cudaFree(g.d_next[b]);
       cudaFreeHost(g.h_order[b]);
       cudaFreeHost(g.h_snap[b]);
       if (g.ev[b] != nullptr) cudaEventDestroy(g.ev[b]);
@@ -681,9 +679,8 @@ void wlg_server::finish_admission(AdmitJob& aj)
       g.team = d.team;
       ok = cuda_ok(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
       for (int b = 0; b < kRing && ok; ++b) {
-        ok = cuda_ok(cudaMalloc(&g.d_order[b], sizeof(int) * static_cast<size_t>(cfg.max_resident))) &&
-             cuda_ok(cudaMalloc(&g.d_next[b], sizeof(int))) &&
-             cuda_ok(cudaMallocHost(&g.h_order[b], sizeof(int) * static_cast<size_t>(cfg.max_resident))) &&
+        ok = cuda_ok(cudaMalloc(&g.d_order[b], sizeof(int) * (static_cast<size_t>(cfg.max_resident) + 1))) &&
+             cuda_ok(cudaMallocHost(&g.h_order[b], sizeof(int) * (static_cast<size_t>(cfg.max_resident) + 1))) &&
              cuda_ok(cudaMallocHost(&g.h_snap[b], sizeof(MainResult) * static_cast<size_t>(cfg.max_resident))) &&
              cuda_ok(cudaEventCreateWithFlags(&g.ev[b], cudaEventDisableTiming));
       }
@@ -740,11 +737,11 @@ bool wlg_server::launch()
       return true;
     }
     const int grid = std::min(cap, (n + per_cta - 1) / per_cta);
-    std::copy(g.members.begin(), g.members.end(), g.h_order[buf]);
-    bool ok = cuda_ok(cudaMemcpyAsync(g.d_order[buf], g.h_order[buf], sizeof(int) * static_cast<size_t>(n),
+    g.h_order[buf][0] = 0;
+    std::copy(g.members.begin(), g.members.end(), g.h_order[buf] + 1);
+    bool ok = cuda_ok(cudaMemcpyAsync(g.d_order[buf], g.h_order[buf], sizeof(int) * (static_cast<size_t>(n) + 1),
                                       cudaMemcpyHostToDevice, g.stream));
-    ok = ok && cuda_ok(cudaMemsetAsync(g.d_next[buf], 0, sizeof(int), g.stream));
-    ok = ok && launch_main_batch(g.form, d_desc, g.d_order[buf], n, g.team, bytes, per_cta, grid, g.d_next[buf],
+    ok = ok && launch_main_batch(g.form, d_desc, g.d_order[buf] + 1, n, g.team, bytes, per_cta, grid, g.d_order[buf],
                                  nullptr, 0, reinterpret_cast<const uint32_t*>(arena_dev),
                                  reinterpret_cast<const uint32_t*>(arena_dev), reinterpret_cast<const int*>(arena_dev),
                                  reinterpret_cast<const uint32_t*>(arena_dev), reinterpret_cast<double*>(arena_dev),
