@@ -75,7 +75,7 @@ __device__ __forceinline__ void pre_problem(const PreDesc& d, unsigned char* sme
   uint32_t* base = reinterpret_cast<uint32_t*>(smem + l.off_base);
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
   uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
-  PreWalk p{X, Y, d.boundary, -2 * N, lg, len, 0, d.n_int, d.len_int, d.n_iter, threads, hist,
+  PreWalk p{X, Y, d.boundary, -2 * N, lg, len, Lh, 0, d.n_int, d.len_int, d.n_iter, threads, hist,
             reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr,
             col, row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words), found_pool + d.off_found};
   const PreSync sync{threads};

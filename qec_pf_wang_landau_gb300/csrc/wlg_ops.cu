@@ -161,7 +161,7 @@ __device__ __forceinline__ void prerun_bonds(const PrerunArgs& a, unsigned char*
   uint32_t* Jr = reinterpret_cast<uint32_t*>(smem + l.off_J);
   uint2* col = reinterpret_cast<uint2*>(smem + l.off_col);
   uint4* row = reinterpret_cast<uint4*>(smem + l.off_row);
-  PreWalk p{X, Y, a.boundary, a.E_min, lg, len, 0, a.n_int, min(a.len_int, 1 << 15), a.n_iter, threads, hist,
+  PreWalk p{X, Y, a.boundary, a.E_min, lg, len, Lh, 0, a.n_int, min(a.len_int, 1 << 15), a.n_iter, threads, hist,
                   reinterpret_cast<uint32_t*>(smem + l.off_claim), reinterpret_cast<int*>(smem + l.off_foundE), thr, col,
                   row, Jr, Jr + X, reinterpret_cast<uint32_t*>(smem + l.off_words),
                   a.found_lat + static_cast<long long>(k) * a.n_int * N};

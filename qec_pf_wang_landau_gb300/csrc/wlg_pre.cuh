@@ -104,10 +104,11 @@ struct PreWalk {
   int X, Y, boundary;
   int e_min, lg;       // lowest energy a walker can have in the range; energies lie 2^lg apart
   int len;             // such energies in the range
+  int stride;          // words from one copy of the histogram to the other, more than len
   int bin0;            // e_min above the first coarse bin's edge
   int n_int, len_int, n_iter;
   int threads;         // walkers, rounded up to a warp
-  uint32_t* hist;      // [2][pre_hist_words(len)], both copies the same
+  uint32_t* hist;      // [2][stride], both copies the same
   uint32_t* claim;     // [n_int]: kPreEmpty, the winner's key, or 0 (stored before the walk)
   int* found_E;        // [n_int] energy of the stored lattice
   const uint32_t* acc_thr;
@@ -191,7 +192,7 @@ __device__ __forceinline__ void pre_walk(const PreWalk& p, const PreSync& sync, 
 {
   constexpr int kW = kTwo ? 2 : 1;
   const int T = p.threads, X = p.X, Y = p.Y, N = X * Y;
-  const int Lh = pre_hist_words(p.len), lg = p.lg;
+  const int Lh = p.stride, lg = p.lg;
   const int spare = Lh - 1;  // takes the visits of threads without a walker
   const uint32_t site_thr = static_cast<uint32_t>(N) * 2048u + 16384u;
   const double site_scale = (N - 1 + 0.999999);
