@@ -246,4 +246,47 @@ inline int kernel_variant(const MainDesc& d, int team, bool resumable)
   return tight_variant(d);
 }
 
+// Threads of one of the teams a problem is spread over.
+inline int rank_team(const MainDesc& d, int ranks) { return round32((d.I + ranks - 1) / ranks * d.W); }
+
+// CTAs a problem is spread over when each may take `spread`: no team smaller than
+// four warps, one per partition of an SM, and a window at least in each.  A team
+// the cluster kernel has no threads for (kClusterThreads; windows of many walkers,
+// or a small spread) leaves the problem on one CTA.
+inline int problem_ranks(const MainDesc& d, int spread)
+{
+  int r = 1;
+  while (r < spread && d.team / (2 * r) >= 128 && d.I >= 2 * r) r *= 2;
+  return rank_team(d, r) <= kClusterThreads ? r : 1;
+}
+
+// The largest spread (up to 8) that leaves every team an SM of its own.  A
+// problem of 512 walkers on one SM has four warps on each partition, which share
+// its issue slots; on four SMs each warp has its own.
+inline int spread_ranks(const Prepared& prep, int sms)
+{
+  int spread = 1;
+  for (int s = 2; s <= 8; s *= 2) {
+    int teams = 0;
+    for (const MainDesc& d : prep.main) teams += problem_ranks(d, s);
+    if (teams <= sms) spread = s;
+  }
+  return spread;
+}
+
+// How run_main launches d: its kernel (a cluster's ranks included) and the
+// threads of a team.  Tight states are not spread.
+struct MainLaunch {
+  int variant, team;
+};
+inline MainLaunch main_launch(const MainDesc& d, int spread, bool resumable)
+{
+  const int ranks = problem_ranks(d, spread);
+  if (ranks > 1) {
+    const int team = rank_team(d, ranks), variant = kernel_variant(d, team, resumable);
+    if ((variant & kVariantTight) == 0) return {variant | ranks * kVariantRanks, team};
+  }
+  return {kernel_variant(d, d.team, resumable), d.team};
+}
+
 }  // namespace wlg

@@ -204,6 +204,10 @@ WLG_HD constexpr bool store_two_words(int store) { return store == kStoreBonds2 
 constexpr int kRingSlots = 16;
 constexpr int kRingWarpBytes = (kRingSlots + 1) * 32 * 4;
 
+// Threads of a CTA that the kernel for problems spread over clusters is compiled
+// for (wlg_main_cluster.cu).
+constexpr int kClusterThreads = 256;
+
 // Energies a proposal can lie beyond its window: one flip changes the energy
 // by at most 8.
 WLG_HD inline int guard_bins(int lg) { return 8 >> lg; }

@@ -720,32 +720,6 @@ namespace {
 // then the histogram (32 bits) [L][team].
 long long pool_slice(int L, int team) { return (3LL * L * team + 1) / 2; }
 
-// CTAs a problem is spread over when each may take `spread`: no team smaller than
-// four warps, one per partition of an SM, and a window at least in each.
-int problem_ranks(const MainDesc& d, int spread)
-{
-  int r = 1;
-  while (r < spread && d.team / (2 * r) >= 128 && d.I >= 2 * r) r *= 2;
-  return r;
-}
-
-// Threads of one of the teams a problem is spread over.
-int rank_team(const MainDesc& d, int ranks) { return round32((d.I + ranks - 1) / ranks * d.W); }
-
-// The largest spread (up to 8) that leaves every team an SM of its own.  A
-// problem of 512 walkers on one SM has four warps on each partition, which share
-// its issue slots; on four SMs each warp has its own.
-int spread_ranks(const Prepared& prep, int sms)
-{
-  int spread = 1;
-  for (int s = 2; s <= 8; s *= 2) {
-    int teams = 0;
-    for (const MainDesc& d : prep.main) teams += problem_ranks(d, s);
-    if (teams <= sms) spread = s;
-  }
-  return spread;
-}
-
 constexpr int kTimedEpoch = 4;  // outer iterations per launch under a time limit
 
 // The main run of a prepared batch: one persistent launch per (variant, team
@@ -777,18 +751,25 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   if (m == 0) return WLG_OK;
   int sms = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex.device);
-  // one launch per (variant, team size) (kernel_variant)
+  // one launch per (variant, team size) (main_launch)
   std::map<std::pair<int, int>, std::vector<int>> groups;
   const bool resumable = time_limit_s > 0;
-  const int spread = resumable ? 1 : spread_ranks(prep, sms);
-  for (int i = 0; i < m; ++i) {
-    const MainDesc& d = prep.main[i];
-    const int ranks = problem_ranks(d, spread), team = rank_team(d, ranks);
-    const int variant = wlg::kernel_variant(d, team, resumable);
-    if (ranks > 1 && (variant & wlg::kVariantTight) == 0) {
-      groups[{variant | ranks * wlg::kVariantRanks, team}].push_back(i);
-    } else {
-      groups[{wlg::kernel_variant(d, d.team, resumable), d.team}].push_back(i);
+  const auto group = [&](int spread) {
+    groups.clear();
+    for (int i = 0; i < m; ++i) {
+      const wlg::MainLaunch l = wlg::main_launch(prep.main[i], spread, resumable);
+      groups[{l.variant, l.team}].push_back(i);
+    }
+  };
+  group(resumable ? 1 : wlg::spread_ranks(prep, sms));
+  // a device that has no room for a cluster (a part of a GPU) runs every problem on one CTA
+  for (const auto& [key, idx] : groups) {
+    if (wlg::variant_ranks(key.first) == 1) continue;
+    int bytes = 0;
+    for (int i : idx) bytes = std::max(bytes, wlg::team_bytes(prep.main[i], key.first, key.second));
+    if (wlg::main_batch_capacity(key.first, key.second, bytes) < wlg::variant_ranks(key.first)) {
+      group(1);
+      break;
     }
   }
   // Longest problems first (larger lattices take more outer iterations of
