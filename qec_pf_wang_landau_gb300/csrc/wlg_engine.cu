@@ -158,6 +158,7 @@ __device__ __forceinline__ void pre_problem_i8(const PreDesc& d, unsigned char* 
   }
   for (int q = tid; q < N; q += blockDim.x) lat[q] = draw_spin(d, q);
   __shared__ uint32_t acc_thr[kAcceptEntries];
+  static_assert(sizeof(acc_thr) <= kPreTableBytes);
   fill_accept(acc_thr, tid);
   __syncthreads();
   const int w = tid;
@@ -261,10 +262,7 @@ wlg_status launch_pre_batch(const PreDesc* d_descs, int n, int threads, int smem
 {
   if (n == 0) return WLG_OK;
   const auto kernel = threads <= 256 ? &k_pre_batch<256> : &k_pre_batch<1024>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return WLG_ERR_CUDA;
-  }
+  if (smem > 48 * 1024 && !allow_shared(kernel, kPreTableBytes)) return WLG_ERR_CUDA;
   kernel<<<n, threads, smem, s>>>(d_descs, n, Jpool, seen_pool, found_pool, fflag_pool);
   return launch_status();
 }
@@ -284,7 +282,7 @@ int main_batch_capacity(int variant, int cta_threads, int smem)
 {
   MainFn fn = main_fn(variant, cta_threads);
   int per_sm = 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
+  if (smem > kSharedBytes || !allow_shared(fn)) return 0;
   const int ranks = variant_ranks(variant);
   if (ranks > 1) {
     cudaLaunchConfig_t cfg{};
@@ -318,7 +316,7 @@ wlg_status launch_main_batch(int variant, const MainDesc* d_descs, const int* d_
   const int threads = team_size * teams_per_cta;
   const int smem = team_bytes * teams_per_cta;
   MainFn fn = main_fn(variant, threads);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return WLG_ERR_CUDA;
+  if (!allow_shared(fn)) return WLG_ERR_CUDA;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));

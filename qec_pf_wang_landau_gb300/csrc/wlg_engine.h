@@ -41,6 +41,7 @@ struct PreDesc {
 // The walk on bond words takes rows of up to 32 sites, 32-bit counts and 22-bit
 // rounds.
 constexpr int kAcceptEntries = 27;
+constexpr int kPreTableBytes = (4 * kAcceptEntries + 15) & ~15;  // static shared memory of the batched pre-run
 WLG_HD inline int pre_hist_words(int len) { return (len + 4) & ~3; }  // one copy, a spare entry included
 // log2 of the distance between a lattice's energies: every site has four bonds
 // (periodic), or some fewer

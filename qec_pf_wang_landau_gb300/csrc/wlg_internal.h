@@ -25,6 +25,20 @@ inline wlg_status cuda_status(cudaError_t e)
   return WLG_ERR_CUDA;
 }
 
+// Shared memory a CTA can have on sm_103.
+constexpr int kSharedBytes = 227 * 1024;
+
+// Lets `kernel`, which has static_bytes of static shared memory, be launched with
+// as much dynamic shared memory as a CTA can have.  The limit is a property of the
+// function that all threads share: always the same value, so that no thread lowers
+// it between another's call and launch.
+template <typename Kernel>
+bool allow_shared(Kernel kernel, int static_bytes = 0)
+{
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes - static_bytes) ==
+         cudaSuccess;
+}
+
 // Runs an entry point's body so that no C++ exception crosses the C ABI:
 // allocation failures become WLG_ERR_OOM, anything else WLG_ERR_INVALID.
 template <typename F>

@@ -995,10 +995,7 @@ wlg_status wlg_wang_landau_pre_run(int* d_energy, int* d_flag_found_interval, in
   }
   cudaStream_t s = as_stream(stream);
   const auto kernel = threads <= 256 ? &k_prerun<256> : &k_prerun<1024>;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-      return WLG_ERR_CUDA;
-  }
+  if (smem > 48 * 1024 && !allow_shared(kernel)) return WLG_ERR_CUDA;
   kernel<<<R, threads, smem, s>>>(a);
   return launch_status();
 }
@@ -1039,9 +1036,7 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
   const int smem = sweep_layout(X, Y, a.L, lg).bytes;
   const auto kernel =
     Y > 16 ? &k_wl_sweep<kStoreRows> : (boundary == 0 ? &k_wl_sweep<kStoreBonds> : &k_wl_sweep<kStoreBondsOpen>);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return WLG_ERR_CUDA;
+  if (smem > 48 * 1024 && !allow_shared(kernel)) return WLG_ERR_CUDA;
   const int samples = (num_lattices + walker_per_sample - 1) / walker_per_sample;
   const int blocks = samples * ((walker_per_sample + 31) / 32);
   kernel<<<blocks, 32 * sweep_warps(blocks), smem, s>>>(a);
