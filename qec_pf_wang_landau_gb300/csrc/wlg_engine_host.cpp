@@ -410,9 +410,13 @@ wlg_status prerun_descs(const wlg_problem* probs, int n, wlg_result* results, Pr
     // a problem is taken when its walk on int8 lattices would fit
     d.smem = wlg::align16(8 * (4 * d.N + 1) + 8 * d.n_int + 16 + 2 * d.N + d.walkers * d.N);
     if (d.smem > 227 * 1024) too_large = true;
-    const int bond_bytes = 
+    // the bond words' state lies beside the kernel's static table
+    const int bond_bytes =
       wlg::pre_layout(d.X, d.Y, (4 * d.N >> wlg::energy_step_log2(d.boundary)) + 1, d.n_int, round32(d.walkers)).bytes;
-    d.bonds = wlg::pre_walk_fits(d.X, d.Y, d.walkers, d.n_iter) && bond_bytes <= 227 * 1024 ? 1 : 0;
+    d.bonds = wlg::pre_walk_fits(d.X, d.Y, d.walkers, d.n_iter) &&
+                      bond_bytes <= wlg::kSharedBytes - wlg::kPreTableBytes
+                ? 1
+                : 0;
     if (d.bonds != 0) d.smem = bond_bytes;
     smem = std::max(smem, d.smem);
     threads = std::max(threads, round32(d.walkers));
