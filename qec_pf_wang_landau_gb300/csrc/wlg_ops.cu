@@ -727,49 +727,64 @@ __global__ void __launch_bounds__(32 * kSweepWarps) k_wl_sweep(const SweepArgs a
 }
 
 // -------------------------------------------------------------- flatness ----
-// wl.cu:892-967, one block per window, a warp per walker: the loads of a
+// wl.cu:892-967, one block per window, 1 to 32 lanes per walker: the loads of a
 // histogram do not wait for each other.
+constexpr int kFlatThreads = 512;  // of a block, at most
+// Lanes a walker: as many as a block has threads for, while all windows' threads
+// are few (a warp's fill whatever they are): beyond, short histograms leave most
+// lanes of a walker idle and the blocks queue.  us for 1 / 32 lanes, 8 bins: 640
+// windows of 16 walkers 5.5 / 13.5, 2560 of 8 8.1 / 21, one of 1024, flat 22 / 144;
+// 120 bins: 16 windows of 8 walkers 24.9 / 5.2.
+inline int flat_lanes(long long windows, int W)
+{
+  int lanes = 32;
+  while (lanes > 1 && (W * lanes > kFlatThreads || (W * lanes > 32 && windows * W * lanes > 65536))) lanes /= 2;
+  return lanes;
+}
 __global__ void k_check_histogram(unsigned long long* __restrict__ H, double* __restrict__ factor,
                                   int8_t* __restrict__ cond, const int* __restrict__ off_hist,
                                   const int* __restrict__ end, const int* __restrict__ start,
                                   const int8_t* __restrict__ spectrum, const int* __restrict__ off_spec,
-                                  const int* __restrict__ cond_inter, double alpha, int W, int wpi, int n_int)
+                                  const int* __restrict__ cond_inter, double alpha, int W, int wpi, int n_int, int lanes)
 {
+  constexpr unsigned kAll = 0xFFFFFFFFu;
   const int b = blockIdx.x;
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int first = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), side = blockDim.x / lanes;
   const int k = (b * W) / wpi;
   if (cond[b] == 1 || cond_inter[k] == -1) return;
   const int len = end[b] - start[b] + 1;
   const int8_t* mask = spectrum + off_spec[k] + start[b] - start[k * n_int];
   bool flat = true;
-  for (int w = threadIdx.x >> 5; w < W && flat; w += warps) {
-    const unsigned long long* h = H + off_hist[b * W + w];
+  for (int w = first; w - first < W && __all_sync(kAll, flat); w += side) {
     unsigned long long mn = 2147483647ull;
     unsigned long long sum = 0;  // exact: the reference's double sum of integers is exact below 2^53
     int cnt = 0;
+    if (w < W) {
+      const unsigned long long* h = H + off_hist[b * W + w];
 #pragma unroll 4
-    for (int i = lane; i < len; i += 32) {
-      const unsigned long long v = h[i];
-      const bool on = mask[i] == 1;
-      mn = on && v < mn ? v : mn;
-      sum += on ? v : 0ull;
-      cnt += on ? 1 : 0;
+      for (int i = lane; i < len; i += lanes) {
+        const unsigned long long v = h[i];
+        const bool on = mask[i] == 1;
+        mn = on && v < mn ? v : mn;
+        sum += on ? v : 0ull;
+        cnt += on ? 1 : 0;
+      }
     }
-    for (int d = 16; d > 0; d >>= 1) {
-      const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, mn, d);
+    for (int d = lanes / 2; d > 0; d >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(kAll, mn, d);
       mn = o < mn ? o : mn;
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
-      cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, d);
+      sum += __shfl_xor_sync(kAll, sum, d);
+      cnt += __shfl_xor_sync(kAll, cnt, d);
     }
     const double avg = static_cast<double>(sum) / max(cnt, 1);
-    flat = cnt > 0 && static_cast<double>(mn) >= alpha * avg;
+    flat = w >= W || (cnt > 0 && static_cast<double>(mn) >= alpha * avg);
   }
   if (!__syncthreads_and(flat)) return;
-  for (int w = threadIdx.x >> 5; w < W; w += warps) {
+  for (int w = first; w < W; w += side) {
     unsigned long long* h = H + off_hist[b * W + w];
-    for (int i = lane; i < len; i += 32) h[i] = 0;
+    for (int i = lane; i < len; i += lanes) h[i] = 0;
+    if (lane == 0) factor[b * W + w] = sqrt(factor[b * W + w]);
   }
-  for (int w = threadIdx.x; w < W; w += blockDim.x) factor[b * W + w] = sqrt(factor[b * W + w]);
   if (threadIdx.x == 0) cond[b] = 1;
 }
 
@@ -1054,9 +1069,11 @@ wlg_status wlg_check_histogram(unsigned long long* d_H, double* d_factor, int8_t
   if (W > 1024 || num_walker_total % W != 0) return WLG_ERR_INVALID;
   const int windows = num_walker_total / W;
   if (windows == 0) return WLG_OK;
-  k_check_histogram<<<windows, std::min(W, 16) * 32, 0, as_stream(stream)>>>(
+  const int lanes = flat_lanes(windows, W);
+  const int threads = std::min((W * lanes + 31) / 32 * 32, kFlatThreads);
+  k_check_histogram<<<windows, threads, 0, as_stream(stream)>>>(
     d_H, d_factor, d_cond, d_offset_histogram, d_end, d_start, d_spectrum, d_offset_spectrum, d_cond_sample, alpha, W,
-    walker_per_sample, num_intervals);
+    walker_per_sample, num_intervals, lanes);
   return launch_status();
 }
 
