@@ -1039,10 +1039,10 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
     // 1 / (1 + overlap (num_intervals - 1)) of it.
     const int full = (4 * N >> lg) + 1;
     a.L = std::min(full, 8 * full / num_intervals + 8);
+    // 2^20 / Y rounded up: e < 32 too large, so that site * e < 4096 * 32 < 2^20
+    // never carries site * magic >> 20 past site / Y
     a.magic = static_cast<uint32_t>(((1u << 20) + Y - 1) / Y);
-    for (int site = 0; site < N; ++site)
-      packed = packed && static_cast<int>((static_cast<uint32_t>(site) * a.magic) >> 20) == site / Y;
-    packed = packed && sweep_layout(X, Y, a.L, lg).bytes <= 227 * 1024;
+    packed = sweep_layout(X, Y, a.L, lg).bytes <= kSharedBytes;
   }
   if (!packed) {
     k_wang_landau<<<blocks_for(static_cast<size_t>(num_lattices)), kThreads, 0, s>>>(a);
