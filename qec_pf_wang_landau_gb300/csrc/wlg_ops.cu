@@ -489,14 +489,41 @@ WLG_HD inline SweepLayout sweep_layout(int X, int Y, int L, int lg)
   return l;
 }
 
-// Warps a block: helpers while all blocks fit beside each other (152 SMs, two
-// blocks of 8 warps each or four of 4 by their registers), one warp beyond,
-// each lane packing its own walker.  1 / 4 / 8 warps, us for 1 and 1000 steps:
-// 10x10, 32 blocks 27 199 / 21 180 / 17 173; 10x10, 512 blocks 40 212 / 25 187 /
-// 33 343 (two waves); 6x6, 1024 blocks 21 211 / 31 324 / 47 619.
-inline int sweep_warps(int blocks)
+// How a call makes its sweep.
+struct SweepPlan {
+  int warps;  // of a block
+  bool pays;  // packed walkers, or the walk on global memory
+};
+// Warps a block: helpers while all blocks fit beside each other (by their registers
+// two blocks of 8 warps on an SM, or four of 4), or where shared memory leaves room
+// for no more; else one warp, each lane packing its own walker.  1 / 4 / 8 warps, us
+// for 1 and 1000 steps: 10x10, 32 blocks 27 199 / 21 180 / 17 173; 10x10, 512 blocks
+// 40 212 / 25 187 / 33 343 (two waves); 6x6, 1024 blocks 21 211 / 31 324 / 47 619.
+// Packing costs a block with 8 warps about 3 us, 36 ns a site and 30 ns a bin of
+// the columns, twice that for each of several waves, and single warps 0.65 ns a site
+// of all blocks together; a step on global memory takes 1 us and more, 1 us per
+// 20 000 walkers.  A sweep whose steps do not make up for the packing stays on
+// global memory.  us of a call, packed / global: 6x6, 15 blocks, 4 steps 14 / 13, 16 steps 17 / 31; 16x16, 256
+// blocks, 8 steps 28 / 22, 32 steps 35 / 58; 32x32, 8 blocks, 8 steps 67 / 21, 64 steps
+// 90 / 112; 10x10, 3200 blocks, 16 steps 222 / 96, 64 steps 241 / 345.
+inline SweepPlan sweep_plan(const SweepArgs& a, int blocks, int bytes)
 {
-  return blocks <= 2 * 152 ? kSweepWarps : (blocks <= 4 * 152 ? kSweepWarps / 2 : 1);
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1)
+    sms = 1;
+  const int room = std::max(kSharedBytes / (bytes + 1024), 1);  // blocks an SM's shared memory holds
+  SweepPlan p{1, false};
+  if (blocks <= 2 * sms || room <= 2) p.warps = kSweepWarps;
+  else if (blocks <= 4 * sms || room <= 4) p.warps = kSweepWarps / 2;
+  const long long beside = static_cast<long long>(sms) * std::min(room, p.warps > 1 ? 16 / p.warps : 16);
+  const long long waves = (blocks + beside - 1) / beside, N = static_cast<long long>(a.X) * a.Y;
+  const long long block_ns = kSweepWarps / p.warps * (3000 + 36 * N + 30ll * a.L);
+  const long long pack_ns = p.warps > 1 ? (waves > 1 ? 2 * waves : 1) * block_ns
+                                        : std::max(13 * N * blocks * 152 / (20ll * sms), (waves - 1) * block_ns);
+  const long long step_ns = std::max(std::max(1000, a.num_lattices / 20) - 200 * (waves - 1), 100ll);
+  p.pays = a.n_iter * step_ns >= pack_ns;
+  return p;
 }
 
 // The sweep of the persistent main run (wlg_sweep.cuh) on the caller's arrays:
@@ -1062,20 +1089,21 @@ wlg_status wlg_wang_landau(int8_t* d_lattice, const int8_t* d_J, unsigned long l
     a.magic = static_cast<uint32_t>(((1u << 20) + Y - 1) / Y);
     packed = sweep_layout(X, Y, a.L, lg).bytes <= kSharedBytes;
   }
-  if (!packed) {
+  const int samples = (num_lattices + walker_per_sample - 1) / walker_per_sample;
+  const int blocks = samples * ((walker_per_sample + 31) / 32);
+  const int smem = packed ? sweep_layout(X, Y, a.L, lg).bytes : 0;
+  const SweepPlan plan = packed ? sweep_plan(a, blocks, smem) : SweepPlan{1, false};
+  if (!plan.pays) {
     k_wang_landau<<<blocks_for(static_cast<size_t>(num_lattices)), kThreads, 0, s>>>(
       d_lattice, d_J, d_H, d_logG, d_factor, d_energy, d_new_energy, d_offset_iter, d_found, d_start, d_end,
       d_offset_histogram, d_offset_lattice, d_cond, d_spectrum, d_offset_spectrum, d_cond_sample, X, Y, num_iterations,
       num_lattices, num_intervals, walker_per_sample, seed, boundary);
     return launch_status();
   }
-  const int smem = sweep_layout(X, Y, a.L, lg).bytes;
   const auto kernel =
     Y > 16 ? &k_wl_sweep<kStoreRows> : (boundary == 0 ? &k_wl_sweep<kStoreBonds> : &k_wl_sweep<kStoreBondsOpen>);
   if (smem > 48 * 1024 && !allow_shared(kernel)) return WLG_ERR_CUDA;
-  const int samples = (num_lattices + walker_per_sample - 1) / walker_per_sample;
-  const int blocks = samples * ((walker_per_sample + 31) / 32);
-  kernel<<<blocks, 32 * sweep_warps(blocks), smem, s>>>(a);
+  kernel<<<blocks, 32 * plan.warps, smem, s>>>(a);
   return launch_status();
 }
 
