@@ -35,6 +35,16 @@ __device__ __forceinline__ size_t divide(size_t t, size_t n)
   return ((t | n) >> 32) == 0 ? static_cast<uint32_t>(t) / static_cast<uint32_t>(n) : t / n;
 }
 
+// SMs of the current device.
+inline int sm_count()
+{
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return 1;
+  return std::max(sms, 1);
+}
+
 // Element t of a sample takes the stream's draw t: a thread takes the four of a
 // Philox block.
 __global__ void k_init_interactions(int8_t* __restrict__ J, size_t N, int R, int seed, float prob)
@@ -343,11 +353,26 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
     for (int q = threadIdx.x; q < 2 * N; q += blockDim.x) fast &= spin(a.J[static_cast<size_t>(k) * 2 * N + q]);
     const unsigned long long most = (1ull << 31) - 1 - static_cast<unsigned long long>(a.n_iter) * a.wpi;
     for (int q = threadIdx.x; q < len; q += blockDim.x) fast &= a.H[static_cast<size_t>(k) * len + q] <= most;
-    if (static_cast<int>(threadIdx.x) < a.wpi) {
-      const size_t t = static_cast<size_t>(k) * a.wpi + threadIdx.x;
+    const int w = threadIdx.x;
+    const size_t t = static_cast<size_t>(k) * a.wpi + w;
+    if constexpr (kMaxThreads > 256) {
+      // More lattices than the L1 cache holds lines for: a warp reads one after
+      // another, 32 sites in one piece (1024 walkers of 24x24 640 -> 78 us; 128
+      // walkers 44 -> 58).
+      const int lane = w & 31, mine = min(32, a.wpi - (w - lane));
+      const long long at = w < a.wpi ? a.off_lat[t] : 0;
+#pragma unroll 4
+      for (int j = 0; j < mine; ++j) {
+        const int8_t* s = a.lat + __shfl_sync(0xFFFFFFFFu, at, j);
+#pragma unroll 4
+        for (int q = lane; q < N; q += 32) fast &= spin(s[q]);
+      }
+    } else if (w < a.wpi) {
       const int8_t* s = a.lat + a.off_lat[t];
 #pragma unroll 16
       for (int q = 0; q < N; ++q) fast &= spin(s[q]);
+    }
+    if (w < a.wpi) {
       fast = fast && (a.seed_off[t] & 1u) == 0;
       // energies on one grid, as the lattices of one sample have them
       fast = fast && ((a.E[t] - a.E[static_cast<size_t>(k) * a.wpi]) & ((1 << energy_step_log2(a.boundary)) - 1)) == 0;
@@ -360,6 +385,22 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_prerun(const PrerunArgs a)
   } else {
     prerun_bonds<true, kMaxThreads <= 256>(a, smem);
   }
+}
+
+// Whether n_iter rounds make up for packing a sample's walkers into bond words.
+// Packing and unpacking cost about 6 us and, per site, 60 ns and what the walkers'
+// strided lattices cost; an int8 round is 1.6 us longer than one on bond words, and
+// 10 ns per walker where there are many.  Samples beyond one an SM wait for each
+// other.  us of a call, bond words / int8: 64 samples of 9x9, 128 walkers, 5 rounds
+// 29 / 27, 20 rounds 32 / 60; 64 of 16x16, 20 rounds 94 / 74, 80 rounds 107 / 194; 2 of
+// 24x24, 1024 walkers, 80 rounds 1446 / 1051, 160 rounds 1615 / 1917; 400 of 16x16, 40
+// rounds 233 / 162, 80 rounds 246 / 287.
+inline bool bonds_pay(long long N, long long walkers, long long n_iter, long long samples)
+{
+  const long long sms = sm_count();
+  const long long pack_ns = (6000 + N * (60 + walkers + walkers * walkers / 1024)) * std::max(samples, sms) / sms;
+  const long long round_ns = std::max(1600ll, 10 * walkers) * std::max(samples, 2 * sms) / (2 * sms);
+  return n_iter * round_ns >= pack_ns;
 }
 
 // ------------------------------------------------------- main WL sweep -----
@@ -508,10 +549,7 @@ struct SweepPlan {
 // 90 / 112; 10x10, 3200 blocks, 16 steps 222 / 96, 64 steps 241 / 345.
 inline SweepPlan sweep_plan(const SweepArgs& a, int blocks, int bytes)
 {
-  int device = 0, sms = 0;
-  if (cudaGetDevice(&device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1)
-    sms = 1;
+  const int sms = sm_count();
   const int room = std::max(kSharedBytes / (bytes + 1024), 1);  // blocks an SM's shared memory holds
   SweepPlan p{1, false};
   if (blocks <= 2 * sms || room <= 2) p.warps = kSweepWarps;
@@ -1045,7 +1083,8 @@ wlg_status wlg_wang_landau_pre_run(int* d_energy, int* d_flag_found_interval, in
   PrerunArgs a{d_energy, d_flag_found_interval, d_lattice, d_found_interval_lattice, d_histogram, d_seed_offset, d_J,
                d_offset_lattice, E_min, E_max, num_iterations, X, Y, seed, static_cast<int>(num_intervals), len_interval,
                walker_per_sample, boundary, 0};
-  if (static_cast<long long>(X) * Y <= 4096 && pre_walk_fits(X, Y, walker_per_sample, num_iterations)) {
+  if (static_cast<long long>(X) * Y <= 4096 && pre_walk_fits(X, Y, walker_per_sample, num_iterations) &&
+      bonds_pay(static_cast<long long>(X) * Y, walker_per_sample, num_iterations, R)) {
     const size_t bytes = static_cast<size_t>(
       pre_layout(X, Y, ((len_hist - 1) >> energy_step_log2(boundary)) + 1, a.n_int, threads).bytes);
     if (bytes <= 227 * 1024) {
