@@ -846,15 +846,17 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   if ((st = ex.buffer(kNext, launches.size() * sizeof(int), &d_next)) != WLG_OK) return st;
   if (timed) cudaMemsetAsync(d_res, 0, static_cast<size_t>(m) * sizeof(MainResult), ex.stream);
   // grids, and the pool of the launches that keep log g and the histogram in
-  // global memory (one slice per resident team, launches side by side; the
+  // global memory: one slice per resident team, launches that run side by side
+  // beside each other, launches that run one after another in the same place (the
   // saved state holds them in resumable runs)
+  const bool in_turn = ex.n_aux == 0;
   std::vector<int> grids(launches.size());
   std::vector<long long> pool_later(launches.size() + 1, 0);  // one CTA's slices of each later launch
   for (size_t g = launches.size(); g-- > 1;) {
     const bool global = (std::get<0>(launches[g]) & wlg::kVariantGlobal) != 0;
     const long long cta = wlg::variant_ranks(std::get<0>(launches[g])) * std::get<3>(launches[g]) *
                           pool_slice(std::get<6>(launches[g]), std::get<1>(launches[g]));
-    pool_later[g - 1] = pool_later[g] + (global ? cta : 0);
+    pool_later[g - 1] = pool_later[g] + (global && !in_turn ? cta : 0);
   }
   std::vector<long long> gpool_off(launches.size(), 0);
   long long gpool_doubles = 0;
@@ -869,12 +871,13 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
       // a fixed arena or a budget may not hold a slice for every team that
       // the GPU could hold: fewer resident teams then take the problems in turn
       const long long slice = pool_slice(Lmax, team);
-      const long long room = static_cast<long long>(ex.available(kGpool) / sizeof(double)) - gpool_doubles;
+      const long long before = in_turn ? 0 : gpool_doubles;
+      const long long room = static_cast<long long>(ex.available(kGpool) / sizeof(double)) - before;
       const long long later = pool_later[g];
       grids[g] = static_cast<int>(std::min<long long>(grids[g], (room - later) / (slice * per_cta)));
       grids[g] = std::max(grids[g] / ranks, 1) * ranks;
-      gpool_off[g] = gpool_doubles;
-      gpool_doubles += grids[g] * per_cta * slice;
+      gpool_off[g] = before;
+      gpool_doubles = std::max(gpool_doubles, before + grids[g] * per_cta * slice);
     }
   }
   void* d_gpool = nullptr;
@@ -1525,8 +1528,9 @@ struct ArenaExec final : Exec {
 // global log g, at most (problems + teams per CTA - 1) times per launch (one
 // launch per team size and lattice layout), for every problem whose full-range
 // state of 16 bytes per bin and walker would not fit shared memory.  The pool
-// that run_main then takes follows the room left (Exec::available); one CTA's
-// slices fit in the part of the arena beyond the admitted bytes.
+// that run_main then takes follows the room left (Exec::available) and is shared by
+// the launches, which run in turn; one CTA's or cluster's slices always fit in the
+// part of the arena beyond the admitted bytes.
 size_t noalloc_bound(const wlg_problem* probs, int n)
 {
   auto pad = [](size_t x) { return (x + 255) & ~size_t{255}; };

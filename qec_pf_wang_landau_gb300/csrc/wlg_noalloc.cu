@@ -22,9 +22,9 @@
 #include "../../include/wlg.h"
 
 namespace wlg {
-// what a batch may need (noalloc_bound), and room for the slices of one CTA
-// per launch of the global log g pool, which the bound counts by an older,
-// smaller slice or not at all
+// what a batch may need (noalloc_bound), and room for the slices of one CTA (340
+// KB) or one cluster (eight times that) of the global log g pool, which the bound
+// counts by an older, smaller slice or not at all
 constexpr size_t kNoAllocAdmitted = size_t{8} << 20;
 constexpr size_t kNoAllocBytes = kNoAllocAdmitted + (size_t{4} << 20);
 size_t noalloc_admitted() { return kNoAllocAdmitted; }
