@@ -285,16 +285,23 @@ struct wlg_context {
 
 namespace {
 
+void release(wlg_context* ctx, DevBuf& b)
+{
+  if (b.p == nullptr) return;
+  cudaFree(b.p);
+  ctx->used -= b.cap;
+  b.p = nullptr;
+  b.cap = 0;
+}
+
 wlg_status grow(wlg_context* ctx, DevBuf& b, size_t bytes, std::string& err)
 {
   if (bytes <= b.cap) return WLG_OK;
   bytes = std::max<size_t>(bytes, 256);
-  if (b.p != nullptr) {
-    cudaFree(b.p);
-    ctx->used -= b.cap;
-    b.p = nullptr;
-    b.cap = 0;
-  }
+  release(ctx, b);
+  // The pool of log g takes what a batch leaves of the budget; it is the last buffer
+  // of a solve, so another one that grows finds an earlier solve's.
+  if (ctx->budget != 0 && ctx->used + bytes > ctx->budget) release(ctx, ctx->buf[kGpool]);
   if (ctx->budget != 0 && ctx->used + bytes > ctx->budget) {
     err = "device memory budget";
     return WLG_ERR_OOM;
