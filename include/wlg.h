@@ -355,10 +355,11 @@ wlg_status wlg_solve_plain(const wlg_problem* problems, int n, wlg_result* resul
  * trajectory is its own).  out[i] (up to cap) describes group i; *n_out =
  * number of groups. */
 typedef struct {
-  int form;        /* main-run form: 0 shared-memory lattice, 1 register lattice, 2 register + table */
+  int form;        /* main-run form: 0 shared-memory lattice, 1 register lattice, 2 register + table,
+                      3 log g in global memory */
   int team;        /* threads per team (walkers, rounded up to a warp) */
   int per_cta;     /* chosen teams per CTA */
-  float main_ms;   /* its main-run time on the capped batch */
+  float main_ms;   /* its main-run time on the capped batch, no problem spread over a cluster */
   int candidates;  /* choices timed */
 } wlg_tuning;
 

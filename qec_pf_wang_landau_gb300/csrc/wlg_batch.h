@@ -80,6 +80,7 @@ struct Exec {
   // teams per CTA chosen by an autotuner, by (form, team size); nullptr or
   // no entry: the built-in rule
   const std::map<std::pair<int, int>, int>* per_cta = nullptr;
+  bool may_spread = true;  // problems over clusters, where SMs are idle
   WorkerPool* pool = nullptr;  // host threads for the per-problem phases; nullptr: the calling thread
   // streams on which the main-run launches of different groups run side by
   // side (fork/join through aux_ev: [0] fork, [1 + a] join of aux[a]);

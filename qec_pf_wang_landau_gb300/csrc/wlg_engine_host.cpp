@@ -772,7 +772,7 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
       groups[{l.variant, l.team}].push_back(i);
     }
   };
-  group(resumable ? 1 : wlg::spread_ranks(prep, sms));
+  group(resumable || !ex.may_spread ? 1 : wlg::spread_ranks(prep, sms));
   // a device that has no room for a cluster (a part of a GPU) runs every problem on one CTA
   for (const auto& [key, idx] : groups) {
     if (wlg::variant_ranks(key.first) == 1) continue;
@@ -1381,7 +1381,9 @@ wlg_status wlg_context_autotune(wlg_context* ctx, const wlg_problem* problems, i
       ctx->err = ex.err;
       return st;
     }
-    // problems by (form, team size), as run_main groups them
+    // problems by (form, team size), as run_main groups those that it does not
+    // spread: teams per CTA are chosen for these alone
+    ex.may_spread = false;
     std::map<std::pair<int, int>, std::vector<int>> groups;
     for (size_t i = 0; i < prep.main.size(); ++i) {
       const MainDesc& d = prep.main[i];
