@@ -83,11 +83,15 @@ struct Exec {
   bool may_spread = true;  // problems over clusters, where SMs are idle
   WorkerPool* pool = nullptr;  // host threads for the per-problem phases; nullptr: the calling thread
   // streams on which the main-run launches of different groups run side by
-  // side (fork/join through aux_ev: [0] fork, [1 + a] join of aux[a]);
-  // n_aux = 0: all on `stream`, one after another
+  // side (fork/join through aux_ev: [0] fork, [1 + a] join of aux[a])
   cudaStream_t* aux = nullptr;
   cudaEvent_t* aux_ev = nullptr;
-  int n_aux = 0;
+  // how many of `wanted` such streams there are; 0: all on `stream`, one after another
+  virtual int side_streams(int wanted)
+  {
+    (void)wanted;
+    return 0;
+  }
   virtual ~Exec() = default;
   // device buffer for `slot` of at least `bytes` bytes
   virtual wlg_status buffer(Slot slot, size_t bytes, void** out) = 0;

@@ -326,11 +326,20 @@ struct ContextExec final : Exec {
     ev = c->ev;
     per_cta = &c->tuned;
     pool = &c->workers();
-    if (c->aux[0] != nullptr) {
-      aux = c->aux;
-      aux_ev = c->aux_ev;
-      n_aux = wlg_context::kAux;
-    }
+    aux = c->aux;
+    aux_ev = c->aux_ev;
+  }
+  // made when a batch first has that many launch groups, and kept
+  int side_streams(int wanted) override
+  {
+    const auto event = [&](int q) {
+      return aux_ev[q] != nullptr || cudaEventCreateWithFlags(&aux_ev[q], cudaEventDisableTiming) == cudaSuccess;
+    };
+    int n = 0;
+    while (n < std::min(wanted, wlg_context::kAux) && event(0) && event(1 + n) &&
+           (aux[n] != nullptr || cudaStreamCreateWithFlags(&aux[n], cudaStreamNonBlocking) == cudaSuccess))
+      ++n;
+    return n;
   }
   wlg_status buffer(Slot slot, size_t bytes, void** out) override
   {
@@ -856,7 +865,8 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
   // global memory: one slice per resident team, launches that run side by side
   // beside each other, launches that run one after another in the same place (the
   // saved state holds them in resumable runs)
-  const bool in_turn = ex.n_aux == 0;
+  const int n_fork = launches.size() > 1 ? ex.side_streams(static_cast<int>(launches.size())) : 0;
+  const bool in_turn = n_fork == 0;
   std::vector<int> grids(launches.size());
   std::vector<long long> pool_later(launches.size() + 1, 0);  // one CTA's slices of each later launch
   for (size_t g = launches.size(); g-- > 1;) {
@@ -895,7 +905,6 @@ wlg_status run_main(Exec& ex, wlg_result* results, Prepared& prep, const Handoff
     cudaMemsetAsync(d_next, 0, launches.size() * sizeof(int), ex.stream);
     // groups side by side: a persistent launch's CTAs exit as its queue
     // drains, and the next group's CTAs take the freed SMs during its tail
-    const int n_fork = ex.n_aux > 0 && launches.size() > 1 ? std::min<int>(ex.n_aux, static_cast<int>(launches.size())) : 0;
     if (n_fork > 0) {
       cudaEventRecord(ex.aux_ev[0], ex.stream);
       for (int a = 0; a < n_fork; ++a) cudaStreamWaitEvent(ex.aux[a], ex.aux_ev[0], 0);
@@ -1057,10 +1066,6 @@ wlg_status wlg_context_create(int device, size_t mem_budget_bytes, wlg_context**
     }
     ctx->stream = ctx->own_stream;
     for (auto& e : ctx->ev) cudaEventCreate(&e);
-    bool aux_ok = true;
-    for (auto& a : ctx->aux) aux_ok = aux_ok && cudaStreamCreateWithFlags(&a, cudaStreamNonBlocking) == cudaSuccess;
-    for (auto& e : ctx->aux_ev) aux_ok = aux_ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    if (!aux_ok) ctx->release_aux();  // launches then run one after another on the context's stream
     *out = ctx;
     return WLG_OK;
   });
