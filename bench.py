@@ -47,7 +47,9 @@ sys.path.insert(0, ROOT)
 WORKLOAD = dict(X=6, Y=6, boundary=0, prob=0.04, seed=12345, samples=100, classes="ivhc", pre_walkers=128,
                 pre_intervals=32, pre_iterations=1000, intervals=10, walkers_per_interval=3, overlap=0.25, alpha=0.8,
                 beta=1e-3, iterations=1000, exchange_every=20)
-BYTES_PER_FLIP = 34  # log g read old + read new + write (24 B), histogram RMW (8 B), packed neighbourhood (~2 B)
+# shared-memory bytes of a step on this workload's lattices (spins in registers): table entry and degree (20 B),
+# bin (8 B read, 4 B written), two draws (8 B read, 8 B written); log g and histogram change once per sweep
+SMEM_BYTES_PER_FLIP = 48
 # DRAM bytes (read + write) of one main-run launch of this workload, from an ncu capture of the
 # bench's own launch (dram__bytes_read.sum + dram__bytes_write.sum); walker state never leaves the SM
 MAIN_TRAFFIC_BYTES = 864256
@@ -823,7 +825,8 @@ def run_ours(args):
     # baseline is a rank-0, N = 1 figure; at N > 1 they would hold every GPU)
     single = ws == 1
     peaks, peak_kind = measured_peaks()
-    achieved = BYTES_PER_FLIP * flips / max(t_main, 1e-12) / 1e9
+    # the main run's DRAM traffic: its bound is one warp's chain of steps, no bandwidth
+    achieved = MAIN_TRAFFIC_BYTES * args.steps * ws / max(t_main, 1e-12) / 1e9
     value = converged / t_dev
     line = {
         "metric": METRIC,
@@ -842,7 +845,7 @@ def run_ours(args):
                    "teams_per_cta": {f"f{t['form']}/t{t['team']}": t["per_cta"] for t in tuning}},
         "e2e": {"value": converged / t_e2e, "unit": "samples/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+        "roofline": {"bound": "latency", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": MAIN_TRAFFIC_BYTES,
                      "peak_kind": peak_kind},
         "flips_per_s": flips / t_main,
@@ -871,7 +874,7 @@ def run_ours(args):
     line["accuracy"] = {"rms": {short[k]: v for k, v in acc["rms"].items()},
                         "cls_ok": {short[k]: v for k, v in acc["class_decisions_equal_exact"].items()},
                         "of": acc["samples"], "sets_ok": acc["engine_sets_exact"]}
-    sec = secondary_ceilings(achieved, flips / t_main)
+    sec = secondary_ceilings(flips / t_main)
     detail = {"plain": {"seconds": plain_s, "kernel_launches": plain_launches,
                         "what": "same 400 problems, reference structure on this engine's operator kernels"},
               "reference_cuda": None if ref_cuda is None else {
@@ -943,14 +946,14 @@ def legs_summary(legs):
     return out
 
 
-def secondary_ceilings(achieved_gbs, flips_per_s):
+def secondary_ceilings(flips_per_s):
     """The rates the WL step depends on besides HBM, measured on this device
-    after the timed region (wlg_measure_peaks): the main run's 34 B per flip
-    against shared-memory bandwidth (the level that holds its walker state),
-    and the step rates that Philox draws (two per step) and FP64 exp + log
+    after the timed region (wlg_measure_peaks): the bytes a step moves in shared
+    memory, where its walker state lies, against that bandwidth, and the step rates that Philox draws (two per step) and FP64 exp + log
     (one each per step in the reference's formulation) would allow alone."""
     import qec_pf_wang_landau_gb300 as wlg
     pk = wlg.measure_peaks(0)
+    achieved_gbs = SMEM_BYTES_PER_FLIP * flips_per_s / 1e9
     fp64_step = 1.0 / (1.0 / pk["exp_f64_per_s"] + 1.0 / pk["log_f64_per_s"])
     return {
         "roofline_smem": {"achieved": achieved_gbs, "peak": pk["smem_gbs"], "unit": "GB/s",

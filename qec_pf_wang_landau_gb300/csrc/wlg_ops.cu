@@ -572,13 +572,12 @@ inline SweepPlan sweep_plan(const SweepArgs& a, int blocks, int bytes)
 // the warps, because these short chains of dependent global loads, not bytes,
 // are what a short sweep spends its time on.
 // The step on global memory is one chain of dependent loads and an FP64 exp,
-// about 2.6 us; here 0.13 us.  With helpers, loads that do not wait for each
-// other and the shadows made while packing, a call of one step took, us: 1024
-// walkers of 10x10 34 -> 17, 8192 of 6x6 23 -> 15; of 200 steps 84 -> 52 and
-// 61 -> 50; 81 920 walkers, 1000 steps: 10x10 599 -> 562, 6x6 411 -> 440.  A run
-// of 16 samples of 6x6 on the operators 5.4 -> 5.0 ms (45 with the step on
-// global memory).
-// Warps with arrays the sweep does not take (couplings or spins other than
+// 1.2 to 2 us with few walkers; here 0.13 us.  With helpers, loads that do not wait
+// for each other and the shadows made while packing, a call of 200 steps took, us:
+// 1024 walkers of 10x10 84 -> 52, 8192 of 6x6 61 -> 50; 81 920 walkers, 1000 steps:
+// 10x10 599 -> 562, 6x6 411 -> 440.  A run of 16 samples of 6x6 on the operators 5.4
+// -> 5.0 ms (45 with the step on global memory).
+// Blocks with arrays the sweep does not take (couplings or spins other than
 // +-1, log g of 2^100 and more, factors below 1, an energy outside its window,
 // windows wider than the columns) walk on global memory.
 template <int kStore>
