@@ -400,9 +400,9 @@ __device__ void run_problem(const TeamHead& head, int p, const Team& team, int t
       auto log_g = [&](int c) { return G[c * P + t]; };
       auto new_energy = [&](int En, int step) {
         misc_all[1] = 1;
-        // reported: the last one found, by step, then by walker
-        atomicMax(new_key, static_cast<unsigned long long>(step) << 32 | static_cast<unsigned long long>(t0 + t) << 16 |
-                             static_cast<unsigned>(En + 32768));
+        // reported: the last one found, by step, and of several the lowest walker's
+        atomicMax(new_key, static_cast<unsigned long long>(step) << 32 |
+                             static_cast<unsigned long long>(0xFFFF - (t0 + t)) << 16 | static_cast<unsigned>(En + 32768));
       };
       // Fold the part's visits into histogram and log g, and with both at
       // hand refresh the shadows and take the flatness counts of
